@@ -1,0 +1,615 @@
+// One-CTA symmetric eigensolvers (FP64 results): the Rayleigh-Ritz problem of the Davidson
+// solver (order <= 32) and the Gram matrices of the truncation (order <= 128), all by
+// cyclic Jacobi with the round-robin (Brent-Luk) ordering: n / 2 disjoint plane rotations a
+// round, n - 1 rounds a sweep.
+//
+// What bounds them: a warp's FP64 instruction takes 65 clocks here, dependent or not, and an
+// SM does 1.6 FP64 multiply-adds a clock (both measured); an FP32 one takes 6, and an SM
+// does 128. A Jacobi round in FP64 is 4 n^2 operations after a scalar chain of about ten,
+// so sweeps in FP64 alone cost 8 to 10 times n - 1 rounds of a microsecond and more. Hence:
+//   - the sweeps run in FP32, on off-diagonal elements of 24 bits and diagonal elements of 48
+//     (two floats, so that the gap between two close eigenvalues survives). Their
+//     eigenvectors, applied to those found so far, are orthonormalised in FP64 by
+//     (V^T V)^(-1/2) = I + E/2 + 3/8 E^2 + 5/16 E^3 + O(E^4), E = I - V^T V (1e-6 to 1e-4, so
+//     the remainder is below FP64 rounding), and A = V^T G V is formed anew. A pass brings
+//     the off-diagonal part down by 1e5 to 1e6: two passes, then one FP64 sweep (or as
+//     many as it takes) to 1e-14 of the norm;
+//   - the matrix is its packed lower triangle, updated in place by 2 x 2 blocks (planes
+//     P < Q), a lane for each row of a block: 2 n^2 operations a round instead of 4 to 6 n^2
+//     on the full matrix, and two barriers;
+//   - a rotation's tangent is taken in FP32 (its error leaves 1e-7 of the element it should
+//     annihilate, which the next sweep meets) and the FP32 cosine and sine are brought to
+//     unit length in FP64 by the series of (1 - h)^(-1/2): no FP64 division or square root.
+// Measured, 20 Gram matrices of Gaussian / graded (1 to 1e-18) spectrum, against FP64 sweeps
+// on the full matrix: order 16 0.48 / 0.85 -> 0.14 / 0.21 ms, 32 2.34 / 3.99 -> 0.35 / 0.66,
+// 64 6.2 / 11.7 -> 1.9 / 3.2, 128 41 / 82 -> 13 / 27, with residuals and orthogonality of 1e-15
+// (6e-15 to 6e-14 before). Rayleigh-Ritz of order 16: 332 -> 121 us cold, 177 -> 92 us warm.
+#include "kernels.cuh"
+
+#include <cmath>
+
+namespace c2g {
+
+namespace {
+
+constexpr int kRrMax = 32;
+static_assert(kBatchedEigMax == kRrMax, "the small kernels share their size");
+
+// element (i, j) of a packed symmetric matrix
+__device__ __forceinline__ int tri(int i, int j) {
+  return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
+}
+__host__ __device__ constexpr int tri_size(int m) { return m * (m + 1) / 2; }
+__host__ __device__ constexpr int even_up(int n) { return n + (n & 1); }
+
+template <typename R>
+struct Planes {  // the rotations of a round
+  R c[kBatchedEigLargeMax / 2], s[kBatchedEigLargeMax / 2];
+  int p[kBatchedEigLargeMax / 2], q[kBatchedEigLargeMax / 2];
+  R red[2][32];
+  R low[kBatchedEigLargeMax];  // FP32: what the diagonal of A leaves of its 48 bits
+  int turned;                  // FP32: a rotation of the sweep was above the fine threshold
+};
+
+// Conversions by the bits of the formats, where a conversion instruction takes as long as
+// an FP64 operation: magnitudes below 2^-126 go to zero, d2f truncates, |x| < 2^127.
+__device__ __forceinline__ float d2f(double x) {
+  const unsigned hi = __double2hiint(x), lo = __double2loint(x), mag = hi & 0x7fffffffu;
+  const unsigned f = ((mag - (896u << 20)) << 3) | (lo >> 29);
+  return __uint_as_float(mag < (897u << 20) ? 0u : (hi & 0x80000000u) | f);
+}
+__device__ __forceinline__ double f2d(float x) {
+  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  const unsigned hi = mag < 0x00800000u ? 0u : (b & 0x80000000u) | ((mag >> 3) + (896u << 20));
+  return __hiloint2double(hi, mag < 0x00800000u ? 0u : mag << 29);
+}
+
+// (c, s) in FP32 of the rotation that annihilates apq; d = aqq - app. Entries of magnitude
+// at most about 1.
+__device__ __forceinline__ void rotation32(float d, float apq, float& c, float& s) {
+  const float tau = __fdividef(d, 2.0f * apq), u = fmaf(tau, tau, 1.0f);
+  const float t = copysignf(__fdividef(1.0f, fabsf(tau) + u * rsqrtf(u)), tau);
+  c = rsqrtf(fmaf(t, t, 1.0f));
+  s = t * c;
+  if (apq == 0.0f || !(fabsf(tau) < 1e18f)) {  // nothing to annihilate, or an angle below 1e-18
+    c = 1.0f;
+    s = 0.0f;
+  }
+}
+__device__ __forceinline__ void rotation64(double app, double aqq, double apq, double& c, double& s) {
+  float cf, sf;
+  rotation32(d2f(aqq - app), d2f(apq), cf, sf);
+  const double x = f2d(cf), y = f2d(sf);
+  const double h = fma(-y, y, fma(-x, x, 1.0));
+  const double w = h * fma(0.375, h, 0.5);
+  c = fma(x, w, x);
+  s = fma(y, w, y);
+}
+
+// hi + lo += x (Knuth's two-sum)
+__device__ __forceinline__ void add_low(float& hi, float& lo, float x) {
+  x += lo;
+  const float s = hi + x, b = s - hi;
+  lo = (hi - (s - b)) + (x - b);
+  hi = s;
+}
+
+// Jacobi sweeps on the packed m x m matrix A (m even, entries of magnitude <= 1 or so; an
+// odd order is padded by a zero row), the rotations applied to the columns of V (rows
+// 0 .. n - 1, column j at V + ld j). FP64: until off(A)^2 <= tol |A|^2. FP32: until off(A)^2 is
+// tol times what it was (or 1e-30 |A|^2), and with `fine` until a sweep turns no plane by
+// more than 1e-3 over an element above 1e-16, so that a cluster of small eigenvalues is
+// resolved as well. All threads of the CTA.
+template <typename R>
+__device__ void jacobi_sweeps(R* A, R* V, int ld, int n, int m, Planes<R>& sh, R tol, int max_sweeps,
+                              bool fine = false) {
+  constexpr bool k32 = sizeof(R) == 4;
+  R goal = R(0);
+  constexpr unsigned kAll = 0xffffffffu;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int npair = m / 2, nrow = npair * (npair - 1);  // rows of the 2 x 2 blocks
+  // this thread's first block row (plane P, partner plane P + k) and their steps; the
+  // columns of V start at the warps after the last one with a block row
+  const int row = tid & 1, e0 = tid >> 1, P0 = e0 % npair, k0 = 1 + e0 / npair;
+  const int dP = (nt / 2) % npair, dk = (nt / 2) / npair;
+  const int busy = ((nrow + 31) & ~31) % nt;
+  const int v0 = tid >= busy ? tid - busy : tid + nt - busy;
+  const int i0 = v0 % n, W0 = v0 / n, dI = nt % n, dW = nt / n;
+  for (int sweep = 0; sweep < max_sweeps; sweep++) {
+    R off = R(0), tot = R(0);
+    for (int i = warp; i < m; i += nw)
+      for (int j = lane; j <= i; j += 32) {
+        const R v = A[i * (i + 1) / 2 + j];
+        if (i == j) tot += v * v;
+        else off += v * v;
+      }
+    off *= R(2);
+    tot += off;
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_down_sync(kAll, off, o);
+      tot += __shfl_down_sync(kAll, tot, o);
+    }
+    if (lane == 0) {
+      sh.red[0][warp] = off;
+      sh.red[1][warp] = tot;
+    }
+    __syncthreads();
+    off = tot = R(0);
+    for (int w = 0; w < nw; w++) {
+      off += sh.red[0][w];
+      tot += sh.red[1][w];
+    }
+    if (sweep == 0) goal = k32 ? fmaxf(tol * off, 1e-30f * tot) : tol * tot;
+    const bool again = k32 && fine && sweep > 0 && sh.turned;
+    __syncthreads();
+    if (!(off > goal) && !again) break;
+    if (tid == 0) sh.turned = 0;
+    for (int r = 0; r < m - 1; r++) {
+      if (tid < npair) {
+        // pos(0) = 0, pos(k) = 1 + (k - 1 - r mod m - 1); pairs (pos(t), pos(m - 1 - t))
+        int a = 0, b = m - 2 - tid - r;
+        if (tid > 0) {
+          a = tid - 1 - r;
+          a += 1 + (a < 0 ? m - 1 : 0);
+        }
+        b += 1 + (b < 0 ? m - 1 : 0);
+        const int p = min(a, b), q = max(a, b);
+        const R app = A[tri(p, p)], aqq = A[tri(q, q)], apq = A[tri(q, p)];
+        R c, s;
+        if constexpr (k32) {
+          rotation32((aqq - app) + (sh.low[q] - sh.low[p]), apq, c, s);
+          if (fine && fabsf(s) > 1e-3f && fabsf(apq) > 1e-16f) sh.turned = 1;
+        } else {
+          rotation64(app, aqq, apq, c, s);
+        }
+        sh.c[tid] = c;
+        sh.s[tid] = s;
+        sh.p[tid] = p;
+        sh.q[tid] = q;
+      }
+      __syncthreads();
+      if (nt - 1 - tid < npair) {  // the planes' own diagonal blocks
+        const int P = nt - 1 - tid;
+        const R c = sh.c[P], s = sh.s[P];
+        if (s != R(0)) {
+          const int p = sh.p[P], q = sh.q[P];
+          if constexpr (k32) {
+            // app - t apq and aqq + t apq as two floats; the element between them is gone
+            const float x = __fdividef(s, c) * A[tri(q, p)];
+            A[tri(q, p)] = 0.0f;
+            add_low(A[tri(p, p)], sh.low[p], -x);
+            add_low(A[tri(q, q)], sh.low[q], x);
+          } else {
+            const R a = A[tri(p, p)], b = A[tri(q, p)], d = A[tri(q, q)];
+            const R x = c * a - s * b, y = c * b - s * d, z = s * a + c * b, w = s * b + c * d;
+            A[tri(p, p)] = c * x - s * y;
+            A[tri(q, p)] = s * x + c * y;
+            A[tri(q, q)] = s * z + c * w;
+          }
+        }
+      }
+      // the 2 x 2 blocks of planes P and P + k (mod npair), each pair of planes once; a
+      // lane holds the block's row `row` and has the other from its neighbour
+      for (int e = tid, P = P0, k = k0; e - lane < nrow; e += nt) {
+        const bool in = e < nrow;
+        const int Q = P + k < npair ? P + k : P + k - npair;
+        R own0 = R(0), own1 = R(0), cp = R(1), sp = R(0), cq = R(1), sq = R(0);
+        int at0 = 0, at1 = 0;
+        if (in) {
+          cp = sh.c[P];
+          sp = sh.s[P];
+          cq = sh.c[Q];
+          sq = sh.s[Q];
+          const int p = row ? sh.q[P] : sh.p[P];
+          at0 = tri(p, sh.p[Q]);
+          at1 = tri(p, sh.q[Q]);
+          own0 = A[at0];
+          own1 = A[at1];
+        }
+        if (__any_sync(kAll, sp != R(0) || sq != R(0))) {
+          const R oth0 = __shfl_xor_sync(kAll, own0, 1), oth1 = __shfl_xor_sync(kAll, own1, 1);
+          const R sr = row ? sp : -sp;
+          const R x = cp * own0 + sr * oth0, y = cp * own1 + sr * oth1;
+          if (in) {
+            A[at0] = cq * x - sq * y;
+            A[at1] = sq * x + cq * y;
+          }
+        }
+        P += dP;
+        k += dk;
+        if (P >= npair) {
+          P -= npair;
+          k++;
+        }
+      }
+      for (int i = i0, P = W0; P < npair;) {
+        const R c = sh.c[P], s = sh.s[P];
+        if (s != R(0)) {
+          R* vp = V + ld * sh.p[P] + i;
+          R* vq = V + ld * sh.q[P] + i;
+          const R x = *vp, y = *vq;
+          *vp = c * x - s * y;
+          *vq = s * x + c * y;
+        }
+        i += dI;
+        P += dW;
+        if (i >= n) {
+          i -= n;
+          P++;
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// f(i, j, sum_{k < n} l(i, k) r(k, j)) for i < rows, j < n (lower: rows = n, only i >= j),
+// 2 x 2 elements a thread. Ends with a barrier.
+template <bool kLower, typename FL, typename FR, typename FO>
+__device__ __forceinline__ void cta_product(int rows, int n, FL l, FR r, FO f) {
+  const int rb = (rows + 1) / 2, cb = (n + 1) / 2;
+  for (int e = threadIdx.x; e < rb * cb; e += blockDim.x) {
+    // a full product's rows are half the matrix apart, so that a warp's columns (l(i, k) =
+    // X[k + ld i], ld odd) fall in different banks
+    const int i0 = kLower ? 2 * (e % rb) : e % rb, j0 = 2 * (e / rb);
+    if (kLower && j0 > i0) continue;
+    const int i1 = min(kLower ? i0 + 1 : i0 + rb, rows - 1), j1 = min(j0 + 1, n - 1);
+    double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+    for (int k = 0; k < n; k++) {
+      const double x = l(i0, k), y = l(i1, k), u = r(k, j0), v = r(k, j1);
+      a = fma(x, u, a);
+      b = fma(x, v, b);
+      c = fma(y, u, c);
+      d = fma(y, v, d);
+    }
+    f(i0, j0, a);
+    if (j1 > j0 && (!kLower || j1 <= i0)) f(i0, j1, b);
+    if (i1 > i0) {
+      f(i1, j0, c);
+      if (j1 > j0) f(i1, j1, d);
+    }
+  }
+  __syncthreads();
+}
+
+// The leading dimension of V: odd, so that a warp reading a row meets no bank twice.
+__host__ __device__ constexpr int v_ld(int n) { return n | 1; }
+
+// V = W (n x n), with a zero column where m > n
+__device__ __forceinline__ void load_v(int n, int m, double* V, const double* W) {
+  for (int e = threadIdx.x; e < n * m; e += blockDim.x) V[e % n + v_ld(n) * (e / n)] = e < n * n ? W[e] : 0.0;
+}
+
+// V (n columns of n, orthonormal to 1e-4 or better) orthonormalised, A = V^T G V for the
+// matrix sc G (n x n). W: n x n scratch.
+__device__ void orthonormal_transform(int n, int m, const double* G, double sc, double* A, double* V, double* W) {
+  __shared__ double diag[kBatchedEigLargeMax];
+  const int tid = threadIdx.x, nt = blockDim.x, ld = v_ld(n);
+  auto lower = [&](const double* X, int i, int j) { return i >= j ? X[i + n * j] : X[j + n * i]; };
+  // E, then E^2 in W's lower triangle, then (V^T V)^(-1/2) above it
+  cta_product<true>(
+      n, n, [&](int i, int k) { return V[k + ld * i]; }, [&](int k, int j) { return V[k + ld * j]; },
+      [&](int i, int j, double v) { A[tri(i, j)] = (i == j ? 1.0 : 0.0) - v; });
+  cta_product<true>(
+      n, n, [&](int i, int k) { return A[tri(i, k)]; }, [&](int k, int j) { return A[tri(k, j)]; },
+      [&](int i, int j, double v) { W[i + n * j] = v; });
+  cta_product<true>(
+      n, n, [&](int i, int k) { return A[tri(i, k)]; }, [&](int k, int j) { return lower(W, k, j); },
+      [&](int i, int j, double v) {
+        const double x = (i == j ? 1.0 : 0.0) + fma(0.5, A[tri(i, j)], fma(0.375, W[i + n * j], 0.3125 * v));
+        if (i == j) diag[i] = x;
+        else W[j + n * i] = x;
+      });
+  for (int e = tid; e < n * n; e += nt) {
+    const int i = e % n, j = e / n;
+    if (j <= i) A[i * (i + 1) / 2 + j] = i == j ? diag[i] : W[j + n * i];
+  }
+  __syncthreads();
+  cta_product<false>(
+      n, n, [&](int i, int k) { return V[i + ld * k]; }, [&](int k, int j) { return A[tri(k, j)]; },
+      [&](int i, int j, double v) { W[i + n * j] = v; });
+  load_v(n, m, V, W);
+  __syncthreads();
+  cta_product<false>(
+      n, n, [&](int i, int k) { return G[i + n * k]; }, [&](int k, int j) { return V[k + ld * j]; },
+      [&](int i, int j, double v) { W[i + n * j] = sc * v; });
+  cta_product<true>(
+      n, n, [&](int i, int k) { return V[k + ld * i]; }, [&](int k, int j) { return W[k + n * j]; },
+      [&](int i, int j, double v) { A[tri(i, j)] = v; });
+  if (m > n)
+    for (int e = tid; e < m; e += nt) A[tri(n, e)] = 0.0;
+  __syncthreads();
+}
+
+// An FP32 pass ends at off(A) 3e-6 times what it was, well above FP32's rounding of a
+// rotated matrix.
+constexpr float kTol32 = 1e-11f;
+constexpr int kSweeps32 = 12;
+constexpr int kPasses32 = 2;
+
+// The eigenproblem of sc G (n x n). In: A = V0^T G V0 packed, W = V0 (n x n, orthonormal) or, with
+// `unit`, V0 = 1 and W not set. Out: the eigenvectors V (n x m, leading
+// dimension v_ld(n)) and A = V^T G V diagonal.
+// During an FP32 pass V's memory holds the FP32 eigenvectors and matrix, and W the FP64
+// eigenvectors, which are then multiplied by half their rows at a time through A's memory.
+__device__ void eigen(int n, int m, bool unit, const double* G, double sc, double* A, double* V, double* W, Planes<float>& shf,
+                      Planes<double>& sh) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  float* Vf = reinterpret_cast<float*>(V);
+  float* Af = Vf + n * m;
+  for (int pass = 0; pass < kPasses32; pass++) {
+    for (int e = tid; e < tri_size(m); e += nt) Af[e] = static_cast<float>(A[e]);
+    for (int e = tid; e < n * m; e += nt) Vf[e] = e % n == e / n ? 1.0f : 0.0f;
+    for (int j = tid; j < m; j += nt) {
+      const double d = A[tri(j, j)];
+      shf.low[j] = static_cast<float>(d - static_cast<double>(static_cast<float>(d)));
+    }
+    __syncthreads();
+    jacobi_sweeps<float>(Af, Vf, n, n, m, shf, kTol32, kSweeps32, pass > 0);
+    if (unit && pass == 0) {
+      for (int e = tid; e < n * n; e += nt) W[e] = Vf[e];
+      __syncthreads();
+    } else {
+      for (int r0 = 0; r0 < n; r0 += m / 2) {
+        const int rows = min(m / 2, n - r0);
+        for (int e = tid; e < rows * n; e += nt) A[e] = W[r0 + e % rows + n * (e / rows)];
+        __syncthreads();
+        cta_product<false>(
+            rows, n, [&](int i, int k) { return A[i + rows * k]; },
+            [&](int k, int j) { return f2d(Vf[k + n * j]); },
+            [&](int i, int j, double v) { W[r0 + i + n * j] = v; });
+      }
+    }
+    load_v(n, m, V, W);
+    __syncthreads();
+    orthonormal_transform(n, m, G, sc, A, V, W);
+    if (pass + 1 < kPasses32) {
+      for (int e = tid; e < n * n; e += nt) W[e] = V[e % n + v_ld(n) * (e / n)];
+      __syncthreads();
+    }
+  }
+  jacobi_sweeps<double>(A, V, v_ld(n), n, m, sh, 1e-28, 30);
+}
+
+// The power of two that brings the largest magnitude to [0.5, 1) (1 for a zero, infinite or
+// NaN matrix). v: this thread's largest magnitude; all threads of the CTA.
+__device__ double unit_scale(double v, double* red) {
+  const int tid = threadIdx.x, nw = blockDim.x >> 5;
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((tid & 31) == 0) red[tid >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+  for (int w = 0; w < nw; w++) v = fmax(v, red[w]);
+  __syncthreads();
+  if (!(v > 0.0) || isinf(v)) return 1.0;
+  return ldexp(1.0, -max(-1000, min(1000, ilogb(v) + 1)));
+}
+
+// The rank of diagonal entry j of A among the n in ascending order (ties by index; the
+// index itself where an entry is NaN, so that the ranks are a permutation).
+__device__ __forceinline__ int ascending_rank(const double* A, int n, int j) {
+  const double lam = A[tri(j, j)];
+  int rk = 0;
+  bool nan = false;
+  for (int k = 0; k < n; k++) {
+    const double o = A[tri(k, k)];
+    rk += (o < lam || (o == lam && k < j)) ? 1 : 0;
+    nan |= isnan(o);
+  }
+  return nan ? j : rk;
+}
+
+// Eigenvalues ascending at base + offE, eigenvectors in descending order at base + offU,
+// each with the sign that makes its largest-magnitude entry (the first one on ties)
+// positive -- the layout launch_reverse_columns produces. A is diagonal, times `scale`.
+__device__ void write_descending(const EigJob& jb, double* base, const double* A, const double* V, double scale,
+                                 int* order) {
+  const int n = jb.n, tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
+  for (int j = tid; j < n; j += blockDim.x) {
+    const int rk = ascending_rank(A, n, j);
+    base[jb.offE + rk] = A[tri(j, j)] / scale;
+    order[n - 1 - rk] = j;
+  }
+  __syncthreads();
+  for (int o = tid >> 5; o < n; o += nw) {
+    const double* col = V + v_ld(n) * order[o];
+    double best = -1.0, v = 0.0;
+    int at = n;
+    for (int i = lane; i < n; i += 32)
+      if (fabs(col[i]) > best) {
+        v = col[i];
+        best = fabs(v);
+        at = i;
+      }
+    for (int d = 16; d > 0; d >>= 1) {
+      const double b2 = __shfl_xor_sync(0xffffffffu, best, d), v2 = __shfl_xor_sync(0xffffffffu, v, d);
+      const int a2 = __shfl_xor_sync(0xffffffffu, at, d);
+      if (b2 > best || (b2 == best && a2 < at)) {
+        best = b2;
+        v = v2;
+        at = a2;
+      }
+    }
+    const double sgn = v < 0.0 ? -1.0 : 1.0;
+    for (int i = lane; i < n; i += 32) base[jb.offU + i + static_cast<int64_t>(n) * o] = sgn * col[i];
+  }
+}
+
+// The Rayleigh-Ritz eigenproblem (CheMPS2/Davidson.cpp:242-276, where the reference calls
+// dsyev on the <= 32 x 32 projected matrix). Warm start (Davidson expansion): the matrix
+// grew by one row and column since the previous call, whose eigenvectors E are still in
+// evecs; the solver starts from diag(E, 1)^T M diag(E, 1), diagonal but for the last row and
+// column, which takes two to three sweeps instead of six to ten.
+constexpr int kRrThreads = 256;
+__global__ void __launch_bounds__(kRrThreads, 1) rr_eig_kernel(const double* __restrict__ mat, int n, int ld,
+                                                            double* __restrict__ evals, double* __restrict__ evecs,
+                                                            int warm) {
+  __shared__ double A[tri_size(kRrMax)], V[kRrMax * v_ld(kRrMax)], W[kRrMax * kRrMax], G[kRrMax * kRrMax];
+  __shared__ Planes<double> sh;
+  __shared__ Planes<float> shf;
+  const int tid = threadIdx.x, m = even_up(n);
+  double big = 0.0;
+  for (int e = tid; e < n * n; e += kRrThreads) big = fmax(big, fabs(mat[e % n + ld * (e / n)]));
+  const double sc = unit_scale(big, sh.red[0]), hs = 0.5 * sc;
+  for (int e = tid; e < n * n; e += kRrThreads) {
+    const int i = e % n, j = e / n;
+    G[e] = hs * mat[i + ld * j] + hs * mat[j + ld * i];
+    W[e] = (warm && i < n - 1 && j < n - 1) ? evecs[i + ld * j] : (i == j ? 1.0 : 0.0);
+  }
+  for (int e = tid; e < tri_size(m); e += kRrThreads) A[e] = 0.0;
+  __syncthreads();
+  if (warm) {
+    cta_product<false>(
+        n, n, [&](int i, int k) { return G[i + n * k]; }, [&](int k, int j) { return W[k + n * j]; }, [&](int i, int j, double v) { V[i + n * j] = v; });
+    cta_product<true>(
+        n, n, [&](int i, int k) { return W[k + n * i]; }, [&](int k, int j) { return V[k + n * j]; },
+        [&](int i, int j, double v) { A[tri(i, j)] = v; });
+  } else {
+    for (int e = tid; e < n * n; e += kRrThreads)
+      if (e % n >= e / n) A[tri(e % n, e / n)] = G[e];
+    __syncthreads();
+  }
+  if (n > 1) {
+    eigen(n, m, !warm, G, 1.0, A, V, W, shf, sh);
+  } else {
+    if (tid == 0) V[0] = 1.0;
+    __syncthreads();
+  }
+  for (int e = tid; e < n * n; e += kRrThreads) {
+    const int i = e % n, j = e / n;
+    const int rk = ascending_rank(A, n, j);
+    if (i == 0) evals[rk] = A[tri(j, j)] / sc;
+    evecs[i + ld * rk] = V[i + v_ld(n) * j];
+  }
+}
+
+// The Gram matrices of the truncation: one CTA each; A, V and W as in eigen().
+__device__ __forceinline__ void gram_eigen(const EigJob& jb, double* base, double* A, double* V, double* W,
+                                           Planes<float>& shf, Planes<double>& sh, int* order) {
+  const int n = jb.n, m = even_up(n), tid = threadIdx.x, nt = blockDim.x;
+  const double* G = base + jb.offG;
+  double big = 0.0;
+  for (int e = tid; e < n * n; e += nt) big = fmax(big, fabs(G[e]));
+  const double sc = unit_scale(big, sh.red[0]), hs = 0.5 * sc;
+  for (int e = tid; e < m * m; e += nt) {
+    const int i = e % m, j = e / m;
+    if (j <= i) A[tri(i, j)] = i < n ? hs * G[i + n * j] + hs * G[j + n * i] : 0.0;
+  }
+  __syncthreads();
+  if (n > 1) {
+    eigen(n, m, true, G, sc, A, V, W, shf, sh);
+  } else {
+    if (tid == 0) V[0] = 1.0;
+    __syncthreads();
+  }
+  write_descending(jb, base, A, V, sc, order);
+}
+
+// order <= kBatchedEigMax
+constexpr int kEigSmallThreads = 512;
+__global__ void __launch_bounds__(kEigSmallThreads, 1) batched_eig_kernel(const EigJob* __restrict__ jobs,
+                                                                       double* __restrict__ base) {
+  constexpr int kN = kBatchedEigMax;
+  __shared__ double A[tri_size(kN)], V[kN * v_ld(kN)], W[kN * kN];
+  __shared__ Planes<double> sh;
+  __shared__ Planes<float> shf;
+  __shared__ int order[kN];
+  gram_eigen(jobs[blockIdx.x], base, A, V, W, shf, sh, order);
+}
+
+// order kBatchedEigMax + 1 .. kBatchedEigLargeMax: A and V in dynamic shared memory, the
+// eigenvectors' slot at offU as W until they are written there
+constexpr int kEigLargeThreads = 512;
+__host__ __device__ constexpr size_t eig_large_bytes(int n) {
+  return sizeof(double) * (static_cast<size_t>(tri_size(even_up(n))) + static_cast<size_t>(even_up(n)) * v_ld(n));
+}
+__global__ void __launch_bounds__(kEigLargeThreads) batched_eig_large_kernel(const EigJob* __restrict__ jobs,
+                                                                             double* __restrict__ base) {
+  extern __shared__ double dyn[];
+  __shared__ Planes<double> sh;
+  __shared__ Planes<float> shf;
+  __shared__ int order[kBatchedEigLargeMax];
+  const EigJob jb = jobs[blockIdx.x];
+  gram_eigen(jb, base, dyn, dyn + tri_size(even_up(jb.n)), base + jb.offU, shf, sh, order);
+}
+
+// Loewdin orthonormaliser of k <= 4 vectors: L = S^-1/2 from the k x k overlap S
+// (CheMPS2/Davidson.cpp:367-381). Serial Jacobi, one thread.
+__global__ void lowdin_kernel(const double* __restrict__ overlap, int k, double* __restrict__ lowdin) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  double a[4][4], v[4][4];
+  for (int i = 0; i < k; i++)
+    for (int j = 0; j < k; j++) {
+      a[i][j] = overlap[i + k * j];
+      v[i][j] = (i == j) ? 1.0 : 0.0;
+    }
+  for (int sweep = 0; sweep < 50; sweep++) {
+    double off = 0.0;
+    for (int i = 0; i < k; i++)
+      for (int j = 0; j < k; j++)
+        if (i != j) off += a[i][j] * a[i][j];
+    if (off < 1e-60) break;
+    for (int p = 0; p < k; p++)
+      for (int q = p + 1; q < k; q++) {
+        if (a[p][q] == 0.0) continue;
+        const double tau = (a[q][q] - a[p][p]) / (2.0 * a[p][q]);
+        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+        const double c = 1.0 / sqrt(1.0 + t * t), s = t * c;
+        for (int j = 0; j < k; j++) {
+          const double x = a[p][j], y = a[q][j];
+          a[p][j] = c * x - s * y;
+          a[q][j] = s * x + c * y;
+        }
+        for (int i = 0; i < k; i++) {
+          const double x = a[i][p], y = a[i][q];
+          a[i][p] = c * x - s * y;
+          a[i][q] = s * x + c * y;
+          const double vx = v[i][p], vy = v[i][q];
+          v[i][p] = c * vx - s * vy;
+          v[i][q] = s * vx + c * vy;
+        }
+      }
+  }
+  double f[4];
+  for (int j = 0; j < k; j++) f[j] = pow(a[j][j], -0.5);
+  for (int i = 0; i < k; i++)
+    for (int j = 0; j < k; j++) {
+      double s = 0.0;
+      for (int l = 0; l < k; l++) s += v[i][l] * f[l] * v[j][l];
+      lowdin[i + k * j] = s;
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_small_eig(double* mat, int n, int ld, double* evals, double* evecs, cudaStream_t stream,
+                             bool warm) {
+  if (n < 1 || n > kRrMax || ld < n) return cudaErrorInvalidValue;
+  rr_eig_kernel<<<1, kRrThreads, 0, stream>>>(mat, n, ld, evals, evecs, warm && n > 1 ? 1 : 0);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_batched_eig(const EigJob* jobs, int njobs, double* base, cudaStream_t stream) {
+  if (njobs <= 0) return cudaSuccess;
+  batched_eig_kernel<<<njobs, kEigSmallThreads, 0, stream>>>(jobs, base);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_batched_eig_large(const EigJob* jobs, int njobs, int nmax, double* base, cudaStream_t stream) {
+  if (njobs <= 0) return cudaSuccess;
+  if (nmax > kBatchedEigLargeMax) return cudaErrorInvalidValue;
+  const size_t bytes = eig_large_bytes(nmax);
+  const cudaError_t e = cudaFuncSetAttribute(batched_eig_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(eig_large_bytes(kBatchedEigLargeMax)));
+  if (e != cudaSuccess) return e;
+  batched_eig_large_kernel<<<njobs, kEigLargeThreads, bytes, stream>>>(jobs, base);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_lowdin(const double* overlap, int k, double* lowdin, cudaStream_t stream) {
+  if (k < 1 || k > 4) return cudaErrorInvalidValue;
+  lowdin_kernel<<<1, 32, 0, stream>>>(overlap, k, lowdin);
+  return cudaGetLastError();
+}
+
+}  // namespace c2g

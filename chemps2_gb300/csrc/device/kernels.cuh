@@ -10,9 +10,9 @@
 //                      tiles are reduced in split order, so results are deterministic.
 //   vector kernels     the Davidson eigensolver's dots, linear combinations and
 //                      preconditioner, with deterministic two-pass reductions.
-//   eigensolvers       one-CTA Jacobi for the <= 32 x 32 Rayleigh-Ritz matrix, and
-//                      batched one-CTA Jacobi for the truncation's Gram matrices up to
-//                      order 128 (FP64).
+//   eigensolvers       one-CTA Jacobi (FP32 passes, FP64 finish; eig.cu) for the <= 32 x 32
+//                      Rayleigh-Ritz matrix, and batched for the truncation's Gram
+//                      matrices up to order 128.
 #pragma once
 
 #include <cstdint>
@@ -259,10 +259,10 @@ struct EigJob {
   int64_t offG, offE, offU;
 };
 cudaError_t launch_batched_eig(const EigJob* jobs, int njobs, double* base, cudaStream_t stream);
-// The same for kBatchedEigMax < n <= kBatchedEigLargeMax: one 512-thread CTA per matrix
-// with the matrix in dynamic shared memory and the eigenvector columns rotated in place
-// in global memory (the Gram matrix's own slot, which the matrix is read from first).
-// nmax: the largest n among the jobs (sizes the shared memory).
+// The same for kBatchedEigMax < n <= kBatchedEigLargeMax: one 512-thread CTA per matrix with
+// the matrix and the eigenvectors in dynamic shared memory; the eigenvectors' slot (offU)
+// is scratch until they are written. nmax: the largest n among the jobs (sizes the shared
+// memory).
 constexpr int kBatchedEigLargeMax = 128;
 cudaError_t launch_batched_eig_large(const EigJob* jobs, int njobs, int nmax, double* base, cudaStream_t stream);
 cudaError_t launch_residual(double* t, const double* u, const double* evals, int64_t n, cudaStream_t stream);

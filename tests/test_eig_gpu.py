@@ -57,3 +57,45 @@ def test_rayleigh_ritz_degenerate_and_timing():
     _, prev = np.linalg.eigh(M2[:31, :31])
     _, _, us_warm = c2g.rayleigh_ritz_eig(M2, prev_evecs=prev, reps=20)
     print(f"rayleigh-ritz n=32: cold {us_cold:.1f} us, warm {us_warm:.1f} us per call")
+
+
+def gram(n, kind, rng):
+    if kind == "graded":  # singular values from 1 to 1e-9, as of a converged state
+        q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+        return (q * np.logspace(0, -18, n)) @ q.T
+    if kind == "deficient":  # half the spectrum is zero
+        x = rng.standard_normal((n, n // 2))
+        return x @ x.T
+    if kind == "degenerate":
+        q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+        return (q * np.repeat(np.arange(1.0, n + 1), 3)[:n]) @ q.T
+    if kind == "zero":
+        return np.zeros((n, n))
+    x = rng.standard_normal((n, n + 3))
+    return x @ x.T * {"tiny": 1e-200, "huge": 1e200}[kind]
+
+
+@pytest.mark.parametrize("kind", ["graded", "deficient", "degenerate", "zero", "tiny", "huge"])
+def test_truncation_eig_spectra(kind):
+    """The truncation's eigensolvers at the edges of both kernels' orders. The bar is that of
+    a backward stable solver with room for the order: 1e-12 of the largest eigenvalue."""
+    import ctypes as C
+
+    rng = np.random.default_rng(11)
+    orders = [2, 3, 31, 32, 33, 34, 63, 64, 95, 127, 128]
+    mats = [0.5 * (g + g.T) for g in (gram(n, kind, rng) for n in orders)]
+    ns = np.array(orders, dtype=np.int32)
+    allm = np.concatenate([g.ravel(order="F") for g in mats])
+    ev, vecs = np.zeros(sum(orders)), np.zeros(allm.size)
+    c2g._check(c2g.load().c2g_truncation_eig(len(orders), ns.ctypes.data_as(C.POINTER(C.c_int)), c2g._dp(allm),
+                                             c2g._dp(ev), c2g._dp(vecs)))
+    oe = ov = 0
+    for n, G in zip(orders, mats):
+        w, U = ev[oe:oe + n], vecs[ov:ov + n * n].reshape((n, n), order="F")
+        top = max(float(np.max(np.abs(G))), 1e-300)
+        scale = max(float(np.linalg.norm(G / top, 2)), 1.0)
+        assert np.max(np.abs(w / top - np.linalg.eigvalsh(G / top))) < 1e-12 * scale, n
+        assert np.all(np.diff(w) >= 0), n
+        assert np.max(np.abs(U.T @ U - np.eye(n))) < 1e-12, n
+        assert np.max(np.abs(U.T @ (G / top) @ U - np.diag(w[::-1] / top))) < 1e-12 * scale, n
+        oe, ov = oe + n, ov + n * n
