@@ -548,7 +548,9 @@ __global__ void lowdin_kernel(const double* __restrict__ overlap, int k, double*
     for (int i = 0; i < k; i++)
       for (int j = 0; j < k; j++)
         if (i != j) off += a[i][j] * a[i][j];
-    if (off < 1e-60) break;
+    double tot = off;
+    for (int i = 0; i < k; i++) tot += a[i][i] * a[i][i];
+    if (!(off > 1e-32 * tot)) break;  // below rounding
     for (int p = 0; p < k; p++)
       for (int q = p + 1; q < k; q++) {
         if (a[p][q] == 0.0) continue;

@@ -224,19 +224,24 @@ inline cudaError_t launch_sandwich_warp(const WarpLaunch& w, const int (&counts)
   return cudaSuccess;
 }
 
-// out[j] = sum_i A[i + lda * j] * x[i] for j < ncol (A has n rows). Uses `partial`
-// (at least ncol * kDotBlocks doubles) as scratch.
+// Summing kernels: `partial` is scratch of kDotScratch doubles, whose entry kDotCounter
+// holds an arrival counter (zero between launches, so zeroed when it is allocated).
 constexpr int kDotBlocks = 152;
 constexpr int kDotThreads = 256;
+constexpr int kDotCounter = kDotBlocks * 32;
+constexpr int kDotScratch = kDotCounter + 32;
+// out[j] = sum_i A[i + lda * j] * x[i] for j < ncol <= 32 (A has n rows)
 cudaError_t launch_multi_dot(const double* A, int64_t lda, int ncol, const double* x, int64_t n, double* partial,
                              double* out, cudaStream_t stream);
+// the same into row and column `row` of the symmetric matrix mxm
+cudaError_t launch_project_row(const double* A, int64_t lda, int ncol, const double* x, int64_t n, double* partial,
+                               double* mxm, int ld, int row, cudaStream_t stream);
+// t -= A coef (1 <= ncol <= 32 columns); out[j] = A[:, j] . t, or with `norm` out[0] = t . t
+cudaError_t launch_subtract(double* t, const double* A, int64_t lda, const double* coef, int ncol, int64_t n,
+                            bool norm, double* partial, double* out, cudaStream_t stream);
 // out[i] = beta * out[i] + sum_j coef[j] * A[i + lda * j]   (coef on the device)
 cudaError_t launch_combine(double* out, double beta, const double* A, int64_t lda, const double* coef, int ncol,
                            int64_t n, cudaStream_t stream);
-// Sum of squares of x, written to out[0]
-cudaError_t launch_norm2(const double* x, int64_t n, double* partial, double* out, cudaStream_t stream);
-// x *= s (scalar on the host)
-cudaError_t launch_scale(double* x, double s, int64_t n, cudaStream_t stream);
 // y += a * x
 cudaError_t launch_axpy(double* y, double a, const double* x, int64_t n, cudaStream_t stream);
 cudaError_t launch_fill(double* x, double v, int64_t n, cudaStream_t stream);
@@ -244,8 +249,7 @@ cudaError_t launch_fill(double* x, double v, int64_t n, cudaStream_t stream);
 // sign making the largest-magnitude entry of each column positive
 cudaError_t launch_reverse_columns(double* dst, const double* src, int rows, int cols, cudaStream_t stream);
 
-// Davidson device steps (CheMPS2/Davidson.cpp). `sc` is a small device scratch of
-// scalars; layout documented in kernels.cu.
+// Davidson device steps (CheMPS2/Davidson.cpp).
 // Eigenvalues ascending in evals[0, n), eigenvectors in the columns of evecs (ld). warm:
 // evecs holds the eigenvectors of the leading (n - 1) x (n - 1) block of mat (the previous
 // call on the same matrix before it grew by one row and column).
@@ -265,14 +269,18 @@ cudaError_t launch_batched_eig(const EigJob* jobs, int njobs, double* base, cuda
 // memory).
 constexpr int kBatchedEigLargeMax = 128;
 cudaError_t launch_batched_eig_large(const EigJob* jobs, int njobs, int nmax, double* base, cudaStream_t stream);
-cudaError_t launch_residual(double* t, const double* u, const double* evals, int64_t n, cudaStream_t stream);
-cudaError_t launch_precond_w(double* w, const double* u, const double* diag, const double* evals, double cutoff,
-                             int64_t n, cudaStream_t stream);
-cudaError_t launch_precond_t(double* t, const double* u, const double* diag, const double* evals,
-                             const double* dots2, double cutoff, int64_t n, cudaStream_t stream);
-cudaError_t launch_neg(double* c, int n, cudaStream_t stream);
-cudaError_t launch_inv_sqrt_scale(double* x, const double* sumsq, int64_t n, cudaStream_t stream);
-cudaError_t launch_mxm_row(double* mxm, int ld, int row, const double* dots, int ncol, cudaStream_t stream);
+// u = V coef, t = HV coef - evals[0] u, out[0] = t . t
+cudaError_t launch_ritz(double* t, double* u, const double* HV, const double* V, int64_t lda, const double* coef,
+                        int ncol, const double* evals, int64_t n, double* partial, double* out, cudaStream_t stream);
+// dots2 = (w . t, w . u) of w = K^-1 u, K = diag - evals[0]
+cudaError_t launch_precond_dots(const double* t, const double* u, const double* diag, const double* evals,
+                                double cutoff, int64_t n, double* partial, double* dots2, cudaStream_t stream);
+// t = -K^-1 (t - dots2[0] / dots2[1] u); out[j] = A[:, j] . t for j < ncol <= 32
+cudaError_t launch_precond(double* t, const double* u, const double* diag, const double* evals, const double* dots2,
+                           double cutoff, const double* A, int64_t lda, int ncol, int64_t n, double* partial,
+                           double* out, cudaStream_t stream);
+// dst = x / sqrt(sumsq[0])
+cudaError_t launch_normalize(double* dst, const double* x, const double* sumsq, int64_t n, cudaStream_t stream);
 cudaError_t launch_lowdin(const double* overlap, int k, double* lowdin, cudaStream_t stream);
 
 }  // namespace c2g

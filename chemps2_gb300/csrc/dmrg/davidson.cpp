@@ -12,7 +12,8 @@ namespace {
 constexpr int kMxM = 0;         // 32 x 32 Rayleigh-Ritz matrix (ld 32)
 constexpr int kEvecs = 1024;    // its eigenvectors (ld 32)
 constexpr int kEvals = 2048;    // eigenvalues, ascending
-constexpr int kDots = 2112;     // up to 64 dot products
+constexpr int kDots = 2112;     // up to 32 dot products
+constexpr int kDotsB = 2144;    // those of the second pass of an orthogonalisation
 constexpr int kDots2 = 2176;    // w.t, w.u
 constexpr int kOverlap = 2184;  // keep x keep overlap
 constexpr int kLowdin = 2200;   // keep x keep Loewdin matrix
@@ -41,7 +42,7 @@ DeviceDavidson::DeviceDavidson(Runtime& rt, int64_t n, int max_vec, int keep, do
     throw std::invalid_argument("Davidson: unsupported number of vectors");
   V_ = rt_.alloc(n_ * max_vec_);
   HV_ = rt_.alloc(n_ * max_vec_);
-  W_ = rt_.alloc(n_ * (3 + keep_));
+  W_ = rt_.alloc(n_ * (2 + keep_));
   sm_ = rt_.alloc(kSmall);
   rt_.zero(sm_, kSmall);
   host_ = rt_.pinned_scalars();
@@ -56,11 +57,15 @@ DeviceDavidson::~DeviceDavidson() {
 
 void DeviceDavidson::multi_dot(const double* A, int ncol, const double* x, double* out) {
   C2G_CUDA(launch_multi_dot(A, n_, ncol, x, n_, rt_.partial(), out, rt_.stream()));
-  count_launches(2);
+  count_launches(1);
 }
 
-double DeviceDavidson::norm2(const double* x, double* theta) {
+double DeviceDavidson::norm2(const double* x) {
   multi_dot(x, 1, x, sm_ + kSumSq);
+  return read_sumsq(nullptr);
+}
+
+double DeviceDavidson::read_sumsq(double* theta) {
   C2G_CUDA(cudaMemcpyAsync(host_, sm_ + kSumSq, sizeof(double), cudaMemcpyDeviceToHost, rt_.stream()));
   if (theta) C2G_CUDA(cudaMemcpyAsync(host_ + 1, sm_ + kEvals, sizeof(double), cudaMemcpyDeviceToHost, rt_.stream()));
   rt_.sync();
@@ -68,19 +73,45 @@ double DeviceDavidson::norm2(const double* x, double* theta) {
   return host_[0];
 }
 
-// CheMPS2/Davidson.cpp:216-236 (AddNewVec): t <- t - V V^T t (twice), t <- t / |t|, V[nv] <- t.
-void DeviceDavidson::add_new_vec(double* t, int nv) {
+// CheMPS2/Davidson.cpp:216-236 (AddNewVec): t <- t - V V^T t (twice), V[nv] <- t / |t|.
+void DeviceDavidson::add_new_vec(double* t, int nv, bool projected) {
   cudaStream_t s = rt_.stream();
-  for (int pass = 0; pass < 2 && nv > 0; pass++) {
-    multi_dot(V_, nv, t, sm_ + kDots);
-    C2G_CUDA(launch_neg(sm_ + kDots, nv, s));
-    C2G_CUDA(launch_combine(t, 1.0, V_, n_, sm_ + kDots, nv, n_, s));
+  double* partial = rt_.partial();
+  if (nv > 0) {
+    if (!projected) multi_dot(V_, nv, t, sm_ + kDots);
+    C2G_CUDA(launch_subtract(t, V_, n_, sm_ + kDots, nv, n_, false, partial, sm_ + kDotsB, s));
+    C2G_CUDA(launch_subtract(t, V_, n_, sm_ + kDotsB, nv, n_, true, partial, sm_ + kSumSq, s));
     count_launches(2);
+  } else {
+    multi_dot(t, 1, t, sm_ + kSumSq);
   }
-  multi_dot(t, 1, t, sm_ + kSumSq);
-  C2G_CUDA(launch_inv_sqrt_scale(t, sm_ + kSumSq, n_, s));
+  C2G_CUDA(launch_normalize(V(nv), t, sm_ + kSumSq, n_, s));
   count_launches(1);
-  C2G_CUDA(cudaMemcpyAsync(V(nv), t, sizeof(double) * n_, cudaMemcpyDeviceToDevice, s));
+}
+
+// DiagonalizeSmallMatrixAndCalcResidual (CheMPS2/Davidson.cpp:238-289) with the newest
+// product HV(nv); returns the residual norm (and, with theta, the lowest Ritz value).
+double DeviceDavidson::ritz(int& nv, double* theta) {
+  cudaStream_t s = rt_.stream();
+  double* partial = rt_.partial();
+  C2G_CUDA(launch_project_row(HV_, n_, nv + 1, V(nv), n_, partial, sm_ + kMxM, kLd, nv, s));
+  nv++;
+  // warm start when the previous solve was of this matrix's leading block
+  C2G_CUDA(launch_small_eig(sm_ + kMxM, nv, kLd, sm_ + kEvals, sm_ + kEvecs, s, eig_n_ == nv - 1));
+  eig_n_ = nv;
+  C2G_CUDA(launch_ritz(W(0), W(1), HV_, V_, n_, sm_ + kEvecs, nv, sm_ + kEvals, n_, partial, sm_ + kSumSq, s));
+  count_launches(3);
+  return std::sqrt(read_sumsq(theta));
+}
+
+// CalculateNewVec (CheMPS2/Davidson.cpp:291-317) into W(0), and its products with V[0..nproj)
+void DeviceDavidson::new_vec(const double* diag, int nproj) {
+  cudaStream_t s = rt_.stream();
+  double* partial = rt_.partial();
+  C2G_CUDA(launch_precond_dots(W(0), W(1), diag, sm_ + kEvals, cutoff_, n_, partial, sm_ + kDots2, s));
+  C2G_CUDA(launch_precond(W(0), W(1), diag, sm_ + kEvals, sm_ + kDots2, cutoff_, V_, n_, nproj, n_, partial,
+                          sm_ + kDots, s));
+  count_launches(2);
 }
 
 bool DeviceDavidson::run(const double* diag, const MatVec& matvec, Precision prec, double tol, bool stop_on_stall,
@@ -88,7 +119,6 @@ bool DeviceDavidson::run(const double* diag, const MatVec& matvec, Precision pre
   cudaStream_t s = rt_.stream();
   double* t = W(0);
   double* u = W(1);
-  double* w = W(2);
   auto mv = [&](const double* x, double* y) {
     matvec(x, y, prec);
     st.n_matvec++;
@@ -102,19 +132,8 @@ bool DeviceDavidson::run(const double* diag, const MatVec& matvec, Precision pre
   int since_best = 0;
   const int matvec0 = st.n_matvec;
   for (;;) {
-    // DiagonalizeSmallMatrixAndCalcResidual (CheMPS2/Davidson.cpp:238-289)
-    multi_dot(HV_, nv + 1, V(nv), sm_ + kDots);
-    C2G_CUDA(launch_mxm_row(sm_ + kMxM, kLd, nv, sm_ + kDots, nv + 1, s));
-    nv++;
-    // warm start when the previous solve was of this matrix's leading block
-    C2G_CUDA(launch_small_eig(sm_ + kMxM, nv, kLd, sm_ + kEvals, sm_ + kEvecs, s, eig_n_ == nv - 1));
-    eig_n_ = nv;
-    C2G_CUDA(launch_combine(t, 0.0, HV_, n_, sm_ + kEvecs, nv, n_, s));
-    C2G_CUDA(launch_combine(u, 0.0, V_, n_, sm_ + kEvecs, nv, n_, s));
-    C2G_CUDA(launch_residual(t, u, sm_ + kEvals, n_, s));
-    count_launches(5);
     double theta = 0.0;
-    const double rnorm = std::sqrt(norm2(t, stop_on_stall ? &theta : nullptr));
+    const double rnorm = ritz(nv, stop_on_stall ? &theta : nullptr);
     st.n_iter++;
     st.rnorm = rnorm;
     if (!(rnorm > tol)) break;
@@ -129,36 +148,33 @@ bool DeviceDavidson::run(const double* diag, const MatVec& matvec, Precision pre
       }
       if (st.n_matvec - matvec0 >= kLoMaxMatvec) return false;
     }
-    // CalculateNewVec (CheMPS2/Davidson.cpp:291-317)
-    C2G_CUDA(launch_precond_w(w, u, diag, sm_ + kEvals, cutoff_, n_, s));
-    multi_dot(W(0), 2, w, sm_ + kDots2);  // w.t, w.u
-    C2G_CUDA(launch_precond_t(t, u, diag, sm_ + kEvals, sm_ + kDots2, cutoff_, n_, s));
-    count_launches(2);
+    // with a deflation next, the basis it is to be orthogonal to does not exist yet
+    const bool projected = nv < max_vec_;
+    new_vec(diag, projected ? nv : 0);
     if (nv == max_vec_) {
       // Deflation (CheMPS2/Davidson.cpp:319-384): keep the lowest keep_ Ritz vectors
-      C2G_CUDA(cudaMemcpyAsync(W(3), u, sizeof(double) * n_, cudaMemcpyDeviceToDevice, s));
+      C2G_CUDA(cudaMemcpyAsync(W(2), u, sizeof(double) * n_, cudaMemcpyDeviceToDevice, s));
       for (int c = 1; c < keep_; c++) {
-        C2G_CUDA(launch_combine(W(3 + c), 0.0, V_, n_, sm_ + kEvecs + kLd * c, nv, n_, s));
+        C2G_CUDA(launch_combine(W(2 + c), 0.0, V_, n_, sm_ + kEvecs + kLd * c, nv, n_, s));
         count_launches(1);
       }
-      for (int c = 0; c < keep_; c++) multi_dot(W(3), keep_, W(3 + c), sm_ + kOverlap + keep_ * c);
+      for (int c = 0; c < keep_; c++) multi_dot(W(2), keep_, W(2 + c), sm_ + kOverlap + keep_ * c);
       C2G_CUDA(launch_lowdin(sm_ + kOverlap, keep_, sm_ + kLowdin, s));
       count_launches(1);
       for (int c = 0; c < keep_; c++) {
-        C2G_CUDA(launch_combine(V(c), 0.0, W(3), n_, sm_ + kLowdin + keep_ * c, keep_, n_, s));
+        C2G_CUDA(launch_combine(V(c), 0.0, W(2), n_, sm_ + kLowdin + keep_ * c, keep_, n_, s));
         count_launches(1);
       }
       for (int c = 0; c < keep_; c++) mv(V(c), HV(c));
       // MxMafterDeflation (CheMPS2/Davidson.cpp:510-536)
       eig_n_ = -1;  // the projected matrix is rebuilt
       for (int j = 0; j < keep_; j++) {
-        multi_dot(V_, j + 1, HV(j), sm_ + kDots);
-        C2G_CUDA(launch_mxm_row(sm_ + kMxM, kLd, j, sm_ + kDots, j + 1, s));
+        C2G_CUDA(launch_project_row(V_, n_, j + 1, HV(j), n_, rt_.partial(), sm_ + kMxM, kLd, j, s));
         count_launches(1);
       }
       nv = keep_;
     }
-    add_new_vec(t, nv);
+    add_new_vec(t, nv, projected);
     mv(V(nv), HV(nv));
   }
   return true;
@@ -166,27 +182,14 @@ bool DeviceDavidson::run(const double* diag, const MatVec& matvec, Precision pre
 
 bool DeviceDavidson::refine_cycle(const double* diag, const MatVec& matvec, double tol, int max_expand, double rel,
                                   DavidsonStats& st, double* r_exact) {
-  cudaStream_t s = rt_.stream();
-  double* t = W(0);
-  double* u = W(1);
-  double* w = W(2);
   int nv = 0;
   eig_n_ = -1;
-  add_new_vec(t, nv);
+  add_new_vec(W(0), nv);
   matvec(V(0), HV(0), Precision::kFP64);
   st.n_matvec++;
   double r0 = 0.0;
   for (int it = 0;; it++) {
-    multi_dot(HV_, nv + 1, V(nv), sm_ + kDots);
-    C2G_CUDA(launch_mxm_row(sm_ + kMxM, kLd, nv, sm_ + kDots, nv + 1, s));
-    nv++;
-    C2G_CUDA(launch_small_eig(sm_ + kMxM, nv, kLd, sm_ + kEvals, sm_ + kEvecs, s, eig_n_ == nv - 1));
-    eig_n_ = nv;
-    C2G_CUDA(launch_combine(t, 0.0, HV_, n_, sm_ + kEvecs, nv, n_, s));
-    C2G_CUDA(launch_combine(u, 0.0, V_, n_, sm_ + kEvecs, nv, n_, s));
-    C2G_CUDA(launch_residual(t, u, sm_ + kEvals, n_, s));
-    count_launches(5);
-    const double rnorm = std::sqrt(norm2(t));
+    const double rnorm = ritz(nv, nullptr);
     st.n_iter++;
     st.rnorm = rnorm;
     if (it == 0) {
@@ -197,11 +200,8 @@ bool DeviceDavidson::refine_cycle(const double* diag, const MatVec& matvec, doub
     } else if (rnorm <= rel * r0 || it >= max_expand || nv >= max_vec_) {
       return false;
     }
-    C2G_CUDA(launch_precond_w(w, u, diag, sm_ + kEvals, cutoff_, n_, s));
-    multi_dot(W(0), 2, w, sm_ + kDots2);
-    C2G_CUDA(launch_precond_t(t, u, diag, sm_ + kEvals, sm_ + kDots2, cutoff_, n_, s));
-    count_launches(2);
-    add_new_vec(t, nv);
+    new_vec(diag, nv);
+    add_new_vec(W(0), nv, true);
     matvec(V(nv), HV(nv), lo_);
     st.n_matvec++;
     st.n_matvec_fp32++;

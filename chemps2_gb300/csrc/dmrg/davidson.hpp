@@ -68,9 +68,13 @@ class DeviceDavidson {
   double* V(int i) { return V_ + n_ * i; }
   double* HV(int i) { return HV_ + n_ * i; }
   double* W(int i) { return W_ + n_ * i; }
-  void add_new_vec(double* t, int nv);  // orthonormalise t against V[0..nv) into V[nv]
-  // synchronising host read of x.x (and, with theta, of the lowest Ritz value)
-  double norm2(const double* x, double* theta = nullptr);
+  // orthonormalise t against V[0..nv) into V[nv]; projected: V[0..nv)^T t is in the scratch
+  void add_new_vec(double* t, int nv, bool projected = false);
+  double ritz(int& nv, double* theta);
+  void new_vec(const double* diag, int nproj);
+  // synchronising host reads: x.x; the last sum of squares (and the lowest Ritz value)
+  double norm2(const double* x);
+  double read_sumsq(double* theta);
   void multi_dot(const double* A, int ncol, const double* x, double* out);
   // One Davidson run from the vector in W(0); the Ritz vector ends in W(1). False when a
   // reduced-precision run (stop_on_stall) met a hard step (a stall far above its
@@ -89,7 +93,7 @@ class DeviceDavidson {
   double rtol_, cutoff_;
   double* V_ = nullptr;
   double* HV_ = nullptr;
-  double* W_ = nullptr;   // columns: 0 t, 1 u, 2 w, 3.. deflation vectors
+  double* W_ = nullptr;   // columns: 0 t, 1 u, 2.. deflation vectors
   double* sm_ = nullptr;  // small device scalars (layout in davidson.cpp)
   double* host_ = nullptr;  // pinned host scalars of the runtime
   HostRand* rand_ = nullptr;

@@ -78,7 +78,8 @@ Runtime::Runtime(int L, int device) : L_(L) {
   host_slots32_.assign(kMaxSlots, nullptr);
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&dev_slots_), sizeof(double*) * kMaxSlots));
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&dev_slots32_), sizeof(float*) * kMaxSlots));
-  C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&partial_), sizeof(double) * (kDotBlocks * 64 + 4096)));
+  C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&partial_), sizeof(double) * kDotScratch));
+  C2G_CUDA(cudaMemset(partial_, 0, sizeof(double) * kDotScratch));
   // tile-scheduler counters of the persistent tensor-core kernels (two per kernel)
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&sched_), sizeof(unsigned int) * 4));
   C2G_CUDA(cudaMemset(sched_, 0, sizeof(unsigned int) * 4));
