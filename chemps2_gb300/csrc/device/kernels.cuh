@@ -2,8 +2,7 @@
 //
 //   block sandwich     every term out += alpha sum_p ratio_p op(A_p) op(B) op(C_p) of a
 //                      task-program stage, by output tiles, in three variants: the team
-//                      kernel for tiles up to 16 x 16 (one launch per row class,
-//                      sandwich_warp.cuh), the two-pass GEMM path for large groups
+//                      kernel for tiles up to 16 x 16 (sandwich_warp.cuh), the two-pass GEMM path for large groups
 //                      (intermediates once, then split-K item sums; sandwich_gemm.cu)
 //                      and, for comparison only, the one-pass cooperative and
 //                      item-parallel kernels. Item sums run in a fixed order and split
@@ -182,46 +181,18 @@ struct WarpLaunch {
   const Group* groups;
   const Term* terms;
   const BatchEntry* entries;
-  const WarpTile* tiles;   // ordered by row class
+  const WarpTile* tiles;   // the heaviest first
   double* partials;
   unsigned int* counters;  // zero between launches
 };
 
-// Kernel of row class R (sandwich_warp_r<R>.cu) over `ntiles` tiles of that class.
-template <int R>
-cudaError_t launch_sandwich_warp_class(const WarpLaunch& w, const WarpTile* tiles, int ntiles, const SlotPtrs& sp,
-                                       cudaStream_t stream, Precision prec);
-extern template cudaError_t launch_sandwich_warp_class<0>(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&,
-                                                          cudaStream_t, Precision);
-extern template cudaError_t launch_sandwich_warp_class<1>(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&,
-                                                          cudaStream_t, Precision);
-extern template cudaError_t launch_sandwich_warp_class<2>(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&,
-                                                          cudaStream_t, Precision);
-extern template cudaError_t launch_sandwich_warp_class<3>(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&,
-                                                          cudaStream_t, Precision);
-extern template cudaError_t launch_sandwich_warp_class<4>(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&,
-                                                          cudaStream_t, Precision);
-extern template cudaError_t launch_sandwich_warp_class<5>(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&,
-                                                          cudaStream_t, Precision);
-
-// The team variant over w.tiles (counts[r] tiles of row class r, in class order); returns
-// the number of kernels launched in *launched.
-inline cudaError_t launch_sandwich_warp(const WarpLaunch& w, const int (&counts)[kWarpRowClasses], const SlotPtrs& sp,
-                                        cudaStream_t stream, Precision prec, int* launched) {
-  using Fn = cudaError_t (*)(const WarpLaunch&, const WarpTile*, int, const SlotPtrs&, cudaStream_t, Precision);
-  static constexpr Fn fns[kWarpRowClasses] = {launch_sandwich_warp_class<0>, launch_sandwich_warp_class<1>,
-                                              launch_sandwich_warp_class<2>, launch_sandwich_warp_class<3>,
-                                              launch_sandwich_warp_class<4>, launch_sandwich_warp_class<5>};
-  *launched = 0;
-  int off = 0;
-  for (int r = 0; r < kWarpRowClasses; r++) {
-    if (counts[r] <= 0) continue;
-    const cudaError_t e = fns[r](w, w.tiles + off, counts[r], sp, stream, prec);
-    if (e != cudaSuccess) return e;
-    off += counts[r];
-    ++*launched;
-  }
-  return cudaSuccess;
+// The team variant over w.tiles.
+cudaError_t launch_sandwich_warp_f64(const WarpLaunch& w, int ntiles, const SlotPtrs& sp, cudaStream_t stream);
+cudaError_t launch_sandwich_warp_f32(const WarpLaunch& w, int ntiles, const SlotPtrs& sp, cudaStream_t stream);
+inline cudaError_t launch_sandwich_warp(const WarpLaunch& w, int ntiles, const SlotPtrs& sp, cudaStream_t stream,
+                                        Precision prec) {
+  return prec == Precision::kFP32 ? launch_sandwich_warp_f32(w, ntiles, sp, stream)
+                                  : launch_sandwich_warp_f64(w, ntiles, sp, stream);
 }
 
 // Summing kernels: `partial` is scratch of kDotScratch doubles, whose entry kDotCounter

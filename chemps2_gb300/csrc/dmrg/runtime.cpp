@@ -745,8 +745,6 @@ std::unique_ptr<DevProgram> Runtime::upload_parts(const Program* parts, size_t n
       });
     };
     // Tile order: the groups with the most work first, row-major within a group.
-    // Team-variant tiles are then grouped by row class (one kernel per class), keeping
-    // that order within a class.
     std::vector<int32_t> order(ng);
     {
       // stable LSD radix sort on the complemented work (descending work, program order
@@ -770,21 +768,12 @@ std::unique_ptr<DevProgram> Runtime::upload_parts(const Program* parts, size_t n
         order.swap(tmp);
       }
     }
-    int64_t per_class[kWarpRowClasses] = {0};
-    for (size_t g = 0; g < ng; g++) {
-      const GroupTiles& gi = info[g];
-      if (gi.kind != 2) continue;
-      for (int i = 0; i < gi.tm; i++)
-        for (int j = 0; j < gi.tn; j++) {
-          const int k = shape_of(gi, i, j);
-          per_class[warp_row_class(warp_class_id(gi.rows[k >> 1], gi.cols[k & 1]))] += gi.nsplit[k];
-        }
-    }
-    int64_t class_at[kWarpRowClasses];
     int64_t nwarp_tiles = 0;
-    for (int c = 0; c < kWarpRowClasses; c++) {
-      class_at[c] = nwarp_tiles;
-      nwarp_tiles += per_class[c];
+    for (const GroupTiles& gi : info) {
+      if (gi.kind != 2) continue;
+      const int64_t nr[2] = {gi.tm - 1, 1}, nc[2] = {gi.tn - 1, 1};
+      for (int k = 0; k < 4; k++)
+        if (present(gi, k)) nwarp_tiles += nr[k >> 1] * nc[k & 1] * gi.nsplit[k];
     }
     {
       std::vector<int32_t> lg;
@@ -823,12 +812,11 @@ std::unique_ptr<DevProgram> Runtime::upload_parts(const Program* parts, size_t n
               wt.counter = static_cast<int32_t>(counter++);
               part_off += static_cast<int64_t>(wt.nsplit) * rows * cols;
             }
-            int64_t& at = class_at[warp_row_class(wt.cls)];
             for (int q = 0; q < wt.nsplit; q++) {
               wt.split = q;
               wt.item0 = (wt.nsplit == 1) ? 0 : splits[gi.bounds[k] + q];
               wt.item1 = (wt.nsplit == 1) ? total : splits[gi.bounds[k] + q + 1];
-              wout[at++] = wt;
+              *wout++ = wt;
             }
           }
       }
@@ -943,7 +931,6 @@ std::unique_ptr<DevProgram> Runtime::upload_parts(const Program* parts, size_t n
     ds.tiles_large =
         static_cast<const TileDesc*>(put(tiles_large[s].data(), sizeof(TileDesc) * tiles_large[s].size()));
     ds.ntiles_warp = static_cast<int>(tiles_warp[s].size());
-    for (const WarpTile& wt : tiles_warp[s]) ds.nwarp[warp_row_class(wt.cls)]++;
     ds.tiles_warp =
         static_cast<const WarpTile*>(put(tiles_warp[s].data(), sizeof(WarpTile) * tiles_warp[s].size()));
     const TwoPass& tp = twopass[s];
@@ -1042,11 +1029,10 @@ void Runtime::launch_stage(const DevProgram& p, const DevStage& ds, const SlotPt
     npass += (ch.njtiles > 0) + (ch.nsmall > 0) + (ch.nstiles > 0);
   }
   C2G_CUDA(launch_sandwich_tiles(ds.groups, ds.terms, p.entries, ds.tiles_large, ds.ntiles_large, sp, stream_, prec));
-  int nw = 0;
   const WarpLaunch wl{ds.groups, ds.terms, p.entries, ds.tiles_warp, partials, counters};
-  C2G_CUDA(launch_sandwich_warp(wl, ds.nwarp, sp, stream_, prec, &nw));
+  C2G_CUDA(launch_sandwich_warp(wl, ds.ntiles_warp, sp, stream_, prec));
   C2G_CUDA(launch_sandwich(ds.groups, ds.terms, p.entries, ds.tiles, ds.ntiles, sp, stream_, prec));
-  count_launches(npass + (ds.ntiles > 0) + (ds.ntiles_large > 0) + nw);
+  count_launches(npass + (ds.ntiles > 0) + (ds.ntiles_large > 0) + (ds.ntiles_warp > 0));
 }
 
 void Runtime::sync() {

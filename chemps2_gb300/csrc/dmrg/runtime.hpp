@@ -35,9 +35,8 @@ struct DevStage {
   const Term* terms = nullptr;
   const TileDesc* tiles = nullptr;        // item-parallel variant
   const TileDesc* tiles_large = nullptr;  // cooperative variant
-  const WarpTile* tiles_warp = nullptr;   // team variant, ordered by row class
+  const WarpTile* tiles_warp = nullptr;   // team variant, the heaviest first
   int ngroups = 0, nterms = 0, ntiles = 0, ntiles_large = 0, ntiles_warp = 0;
-  int nwarp[kWarpRowClasses] = {};        // team-variant tiles per row class
   // two-pass path of large groups: pass-1 jobs and tiles, pass-2 groups, items and tiles
   const InterJob* jobs = nullptr;
   const GemmTile* jtiles = nullptr;
