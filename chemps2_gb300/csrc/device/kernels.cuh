@@ -207,6 +207,9 @@ cudaError_t launch_multi_dot(const double* A, int64_t lda, int ncol, const doubl
 // the same into row and column `row` of the symmetric matrix mxm
 cudaError_t launch_project_row(const double* A, int64_t lda, int ncol, const double* x, int64_t n, double* partial,
                                double* mxm, int ld, int row, cudaStream_t stream);
+// out[0] = the lowest diag[i] over the entries with x[i] != 0 (inf: there are none)
+cudaError_t launch_lowest_entry(const double* diag, const double* x, int64_t n, double* partial, double* out,
+                                cudaStream_t stream);
 // t -= A coef (1 <= ncol <= 32 columns); out[j] = A[:, j] . t, or with `norm` out[0] = t . t
 cudaError_t launch_subtract(double* t, const double* A, int64_t lda, const double* coef, int ncol, int64_t n,
                             bool norm, double* partial, double* out, cudaStream_t stream);

@@ -1,6 +1,8 @@
 // Vector kernels of the Davidson eigensolver (FP64, deterministic reductions).
 #include "kernels.cuh"
 
+#include <math_constants.h>
+
 #include <cmath>
 
 namespace c2g {
@@ -103,6 +105,44 @@ __global__ void __launch_bounds__(kDotThreads) multi_dot_kernel(const double* __
   }
   double v;
   if (grid_columns<C>(acc, ncol, partial, counter, v) && threadIdx.x < ncol) o.put(threadIdx.x, v);
+}
+
+// out[0] = the lowest diag[i] over x[i] != 0 (inf if there is none)
+__global__ void __launch_bounds__(kDotThreads) lowest_entry_kernel(const double* __restrict__ diag,
+                                                                   const double* __restrict__ x, int64_t n,
+                                                                   double* partial, unsigned int* counter,
+                                                                   double* out) {
+  constexpr int kWarps = kDotThreads / 32;
+  __shared__ double red[kWarps];
+  __shared__ unsigned int last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double v = CUDART_INF;
+  auto block = [&] {  // the CTA's lowest, in thread 0
+    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (lane == 0) red[warp] = v;
+    __syncthreads();
+    if (tid == 0)
+      for (int w = 1; w < kWarps; w++) v = fmin(v, red[w]);
+  };
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(kDotThreads) + tid; i < n;
+       i += static_cast<int64_t>(gridDim.x) * kDotThreads)
+    if (x[i] != 0.0) v = fmin(v, diag[i]);
+  block();
+  if (tid == 0) {
+    __stcg(partial + blockIdx.x, v);
+    __threadfence();
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v = CUDART_INF;
+  for (int b = tid; b < static_cast<int>(gridDim.x); b += kDotThreads) v = fmin(v, __ldcg(partial + b));
+  block();
+  if (tid == 0) {
+    out[0] = v;
+    *counter = 0u;
+  }
 }
 
 // t -= A coef, then out[j] = A[:, j] . t (kNorm: out[0] = t . t instead)
@@ -337,6 +377,12 @@ cudaError_t launch_multi_dot(const double* A, int64_t lda, int ncol, const doubl
 cudaError_t launch_project_row(const double* A, int64_t lda, int ncol, const double* x, int64_t n, double* partial,
                                double* mxm, int ld, int row, cudaStream_t stream) {
   return dots_into(A, lda, ncol, x, n, partial, SumOut{nullptr, mxm, ld, row}, stream);
+}
+
+cudaError_t launch_lowest_entry(const double* diag, const double* x, int64_t n, double* partial, double* out,
+                                cudaStream_t stream) {
+  lowest_entry_kernel<<<dot_grid(n), kDotThreads, 0, stream>>>(diag, x, n, partial, dot_counter(partial), out);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_subtract(double* t, const double* A, int64_t lda, const double* coef, int ncol, int64_t n,

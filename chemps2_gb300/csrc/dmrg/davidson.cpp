@@ -18,6 +18,7 @@ constexpr int kDots2 = 2176;    // w.t, w.u
 constexpr int kOverlap = 2184;  // keep x keep overlap
 constexpr int kLowdin = 2200;   // keep x keep Loewdin matrix
 constexpr int kSumSq = 2216;    // one sum of squares
+constexpr int kLowest = 2217;   // lowest diagonal entry
 constexpr int kSmall = 2304;
 constexpr int kLd = 32;
 // Mixed-precision refinement: cycles, FP32 expansions per cycle, and the residual
@@ -31,7 +32,9 @@ constexpr double kRefineRel = 1e-3;
 // a poor guess (the first sweep from a random start), on which the FP64 solver may still
 // turn to a lower eigenpair after many more products while the reduced-precision one
 // settles on an excited state. Such a step, and one that needs more than kLoMaxMatvec
-// reduced-precision products, is solved by the FP64 solver from the guess.
+// reduced-precision products, is solved by the FP64 solver from the guess. So is one whose
+// reduced-precision Ritz value ends above a diagonal entry, where no lowest eigenvalue is:
+// the eigenpair found from such a guess hangs on the arithmetic, and the FP64 mode's is meant.
 constexpr double kStallCeiling = 1e-3;
 constexpr int kLoMaxMatvec = 1000;
 }  // namespace
@@ -71,6 +74,18 @@ double DeviceDavidson::read_sumsq(double* theta) {
   rt_.sync();
   if (theta) *theta = host_[1];
   return host_[0];
+}
+
+// The Ritz value is above the lowest diag entry of guess's support by more than its residual
+bool DeviceDavidson::above_diag(const double* diag, const double* guess, double rnorm) {
+  if (partial_diag_) return false;
+  cudaStream_t s = rt_.stream();
+  C2G_CUDA(launch_lowest_entry(diag, guess, n_, rt_.partial(), sm_ + kLowest, s));
+  count_launches(1);
+  C2G_CUDA(cudaMemcpyAsync(host_, sm_ + kLowest, sizeof(double), cudaMemcpyDeviceToHost, s));
+  C2G_CUDA(cudaMemcpyAsync(host_ + 1, sm_ + kEvals, sizeof(double), cudaMemcpyDeviceToHost, s));
+  rt_.sync();
+  return host_[1] > host_[0] + rnorm;
 }
 
 // CheMPS2/Davidson.cpp:216-236 (AddNewVec): t <- t - V V^T t (twice), V[nv] <- t / |t|.
@@ -233,15 +248,11 @@ DavidsonStats DeviceDavidson::solve(double* guess, const double* diag, const Mat
     const bool lo_done = run(diag, matvec, lo_, std::max(lo_tol, rtol_), true, st);
     st.n_lo = st.n_matvec;
     st.lo_rnorm = st.rnorm;
-    if (!lo_done) {  // a hard step: the FP64 solver from the guess
+    if (!lo_done || above_diag(diag, guess, st.rnorm)) {  // a hard step: the FP64 solver from the guess
       st.fp64_fallback = true;
       C2G_CUDA(cudaMemcpyAsync(t, guess, sizeof(double) * n_, cudaMemcpyDeviceToDevice, s));
       run(diag, matvec, Precision::kFP64, rtol_, false, st);
-      C2G_CUDA(cudaMemcpyAsync(guess, u, sizeof(double) * n_, cudaMemcpyDeviceToDevice, s));
-      C2G_CUDA(cudaMemcpyAsync(host_, sm_ + kEvals, sizeof(double), cudaMemcpyDeviceToHost, s));
-      rt_.sync();
-      st.energy = host_[0];
-      return st;
+      done = true;
     }
     // refinement cycles from the FP32 Ritz vector; a cycle that cannot improve (for
     // example an FP32 floor above the target) leaves it to the FP64 Davidson below

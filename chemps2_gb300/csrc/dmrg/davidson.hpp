@@ -59,6 +59,8 @@ class DeviceDavidson {
                       double lo_tol = 1e-5, Precision lo = Precision::kFP32);
   // source of the random start that replaces a zero guess (the C library's rand() unless set)
   void set_rand(HostRand* r) { rand_ = r; }
+  // the matvec adds terms that diag leaves out: its entries bound no eigenvalue
+  void set_partial_diag(bool p) { partial_diag_ = p; }
 
  private:
   Precision lo_ = Precision::kFP32;
@@ -72,6 +74,7 @@ class DeviceDavidson {
   void add_new_vec(double* t, int nv, bool projected = false);
   double ritz(int& nv, double* theta);
   void new_vec(const double* diag, int nproj);
+  bool above_diag(const double* diag, const double* guess, double rnorm);
   // synchronising host reads: x.x; the last sum of squares (and the lowest Ritz value)
   double norm2(const double* x);
   double read_sumsq(double* theta);
@@ -97,6 +100,7 @@ class DeviceDavidson {
   double* sm_ = nullptr;  // small device scalars (layout in davidson.cpp)
   double* host_ = nullptr;  // pinned host scalars of the runtime
   HostRand* rand_ = nullptr;
+  bool partial_diag_ = false;
 };
 
 }  // namespace c2g

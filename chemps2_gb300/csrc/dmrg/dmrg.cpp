@@ -935,6 +935,7 @@ double DMRG::solve_site(const int index, const double dvdson_rtol, const double 
     C2G_CUDA(cudaEventRecord(e1, s));
     timed = true;
   };
+  dav.set_partial_diag(nexc > 0);  // the projectors of the lower states are not in diag
   if (precision_ != 0) ensure_f32(index);
   const c2g::DavidsonStats ds =
       dav.solve(svec, diag, matvec, precision_ != 0, mixed_tol_, matvec_precision(precision_ == 0 ? 1 : precision_));
