@@ -5,25 +5,30 @@
 //
 // What bounds them: a warp's FP64 instruction takes 65 clocks here, dependent or not, and an
 // SM does 1.6 FP64 multiply-adds a clock (both measured); an FP32 one takes 6, and an SM
-// does 128. A Jacobi round in FP64 is 4 n^2 operations after a scalar chain of about ten,
-// so sweeps in FP64 alone cost 8 to 10 times n - 1 rounds of a microsecond and more. Hence:
-//   - the sweeps run in FP32, on off-diagonal elements of 24 bits and diagonal elements of 48
-//     (two floats, so that the gap between two close eigenvalues survives). Their
-//     eigenvectors, applied to those found so far, are orthonormalised in FP64 by
+// does 128. Hence:
+//   - the matrix is its packed lower triangle, updated in place by 2 x 2 blocks (planes
+//     P < Q), a lane for each block, and two barriers a round;
+//   - a rotation is three shears by tan(angle / 2) and sin(angle): three multiply-adds for a
+//     pair of elements instead of four operations;
+//   - the half tangent is taken in FP32 (its error leaves 1e-7 of the element it should
+//     annihilate, which the next sweep meets) and its sine in FP64, from an FP32 reciprocal
+//     and one third-order step: orthogonal to FP64 accuracy, no FP64 division or square root;
+//   - a plane's own diagonal block is updated by differences whose rounding scales with the
+//     angle, so that the off-diagonal part goes on falling to 1e-15 of the norm;
+//   - the Rayleigh-Ritz sweeps run in FP32, on off-diagonal elements of 24 bits and diagonal
+//     elements of 48 (two floats, so that the gap between two close eigenvalues survives).
+//     Their eigenvectors, applied to those found so far, are orthonormalised in FP64 by
 //     (V^T V)^(-1/2) = I + E/2 + 3/8 E^2 + 5/16 E^3 + O(E^4), E = I - V^T V (1e-6 to 1e-4, so
 //     the remainder is below FP64 rounding), and A = V^T G V is formed anew. A pass brings
 //     the off-diagonal part down by 1e5 to 1e6: two passes, then one FP64 sweep (or as
-//     many as it takes) to 1e-14 of the norm;
-//   - the matrix is its packed lower triangle, updated in place by 2 x 2 blocks (planes
-//     P < Q), a lane for each row of a block: 2 n^2 operations a round instead of 4 to 6 n^2
-//     on the full matrix, and two barriers;
-//   - a rotation's tangent is taken in FP32 (its error leaves 1e-7 of the element it should
-//     annihilate, which the next sweep meets) and the FP32 cosine and sine are brought to
-//     unit length in FP64 by the series of (1 - h)^(-1/2): no FP64 division or square root.
+//     many as it takes) to 1e-14 of the norm. The Gram matrices take FP64 sweeps only (see
+//     gram_eigen): the FP32 passes gave 0.35 / 0.66 ms at order 32 and 13 / 27 at 128 in the
+//     table below, but round small eigenvalues to 1e-16 of the norm.
 // Measured, 20 Gram matrices of Gaussian / graded (1 to 1e-18) spectrum, against FP64 sweeps
-// on the full matrix: order 16 0.48 / 0.85 -> 0.14 / 0.21 ms, 32 2.34 / 3.99 -> 0.35 / 0.66,
-// 64 6.2 / 11.7 -> 1.9 / 3.2, 128 41 / 82 -> 13 / 27, with residuals and orthogonality of 1e-15
-// (6e-15 to 6e-14 before). Rayleigh-Ritz of order 16: 332 -> 121 us cold, 177 -> 92 us warm.
+// of four operations on the full matrix: order 16 0.48 / 0.85 -> 0.17 / 0.29 ms, 32 2.34 / 3.99
+// -> 0.53 / 0.92, 64 6.2 / 11.7 -> 2.9 / 5.6, 128 41 / 82 -> 21 / 47, with errors of the
+// eigenvalues and the orthogonality of 0.3 to 2.6e-15 (2 to 70e-15 before). Rayleigh-Ritz
+// of order 16: 332 -> 121 us cold, 177 -> 92 us warm; 32: 982 -> 357 and 584 -> 269.
 #include "kernels.cuh"
 
 #include <cmath>
@@ -43,12 +48,13 @@ __host__ __device__ constexpr int tri_size(int m) { return m * (m + 1) / 2; }
 __host__ __device__ constexpr int even_up(int n) { return n + (n & 1); }
 
 template <typename R>
-struct Planes {  // the rotations of a round
-  R c[kBatchedEigLargeMax / 2], s[kBatchedEigLargeMax / 2];
+struct Planes {  // the rotations of a round: tan(angle / 2) and sin(angle)
+  R h[kBatchedEigLargeMax / 2], s[kBatchedEigLargeMax / 2];
   int p[kBatchedEigLargeMax / 2], q[kBatchedEigLargeMax / 2];
   R red[2][32];
-  R low[kBatchedEigLargeMax];  // FP32: what the diagonal of A leaves of its 48 bits
-  int turned;                  // FP32: a rotation of the sweep was above the fine threshold
+  float tan[kBatchedEigLargeMax / 2];  // FP32: tan(angle)
+  R low[kBatchedEigLargeMax];          // FP32: what the diagonal of A leaves of its 48 bits
+  int turned;                          // FP32: a rotation of the sweep was above the fine threshold
 };
 
 // Conversions by the bits of the formats, where a conversion instruction takes as long as
@@ -64,26 +70,35 @@ __device__ __forceinline__ double f2d(float x) {
   return __hiloint2double(hi, mag < 0x00800000u ? 0u : mag << 29);
 }
 
-// (c, s) in FP32 of the rotation that annihilates apq; d = aqq - app. Entries of magnitude
-// at most about 1.
-__device__ __forceinline__ void rotation32(float d, float apq, float& c, float& s) {
+// The rotation that annihilates apq, d = aqq - app, as h = tan(angle / 2) in FP32 (t:
+// tan(angle)). Entries of magnitude at most about 1.
+__device__ __forceinline__ float half_tangent(float d, float apq, float& t) {
   const float tau = __fdividef(d, 2.0f * apq), u = fmaf(tau, tau, 1.0f);
-  const float t = copysignf(__fdividef(1.0f, fabsf(tau) + u * rsqrtf(u)), tau);
-  c = rsqrtf(fmaf(t, t, 1.0f));
-  s = t * c;
+  t = copysignf(__fdividef(1.0f, fabsf(tau) + u * rsqrtf(u)), tau);
+  const float w = fmaf(t, t, 1.0f);
+  const float h = __fdividef(t, 1.0f + w * rsqrtf(w));
   if (apq == 0.0f || !(fabsf(tau) < 1e18f)) {  // nothing to annihilate, or an angle below 1e-18
-    c = 1.0f;
-    s = 0.0f;
+    t = 0.0f;
+    return 0.0f;
   }
+  return h;
 }
-__device__ __forceinline__ void rotation64(double app, double aqq, double apq, double& c, double& s) {
-  float cf, sf;
-  rotation32(d2f(aqq - app), d2f(apq), cf, sf);
-  const double x = f2d(cf), y = f2d(sf);
-  const double h = fma(-y, y, fma(-x, x, 1.0));
-  const double w = h * fma(0.375, h, 0.5);
-  c = fma(x, w, x);
-  s = fma(y, w, y);
+// sin(angle) = 2 h / (1 + h^2): in FP64 with one third-order step from an FP32 reciprocal, so
+// that the rotation is orthogonal to FP64 accuracy for the h it is given
+__device__ __forceinline__ float sine(float h) { return __fdividef(2.0f * h, fmaf(h, h, 1.0f)); }
+__device__ __forceinline__ double sine(double h, float hf) {
+  const double u = fma(h, h, 1.0);
+  const double r = f2d(__fdividef(1.0f, fmaf(hf, hf, 1.0f)));
+  const double e = fma(-u, r, 1.0);
+  return 2.0 * h * fma(r, fma(e, e, e), r);
+}
+
+// (x, y) <- (c x - s y, s x + c y) by three shears
+template <typename R>
+__device__ __forceinline__ void rotate(R h, R s, R& x, R& y) {
+  x = fma(-h, y, x);
+  y = fma(s, x, y);
+  x = fma(-h, y, x);
 }
 
 // hi + lo += x (Knuth's two-sum)
@@ -107,12 +122,11 @@ __device__ void jacobi_sweeps(R* A, R* V, int ld, int n, int m, Planes<R>& sh, R
   R goal = R(0);
   constexpr unsigned kAll = 0xffffffffu;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  const int npair = m / 2, nrow = npair * (npair - 1);  // rows of the 2 x 2 blocks
-  // this thread's first block row (plane P, partner plane P + k) and their steps; the
-  // columns of V start at the warps after the last one with a block row
-  const int row = tid & 1, e0 = tid >> 1, P0 = e0 % npair, k0 = 1 + e0 / npair;
-  const int dP = (nt / 2) % npair, dk = (nt / 2) / npair;
-  const int busy = ((nrow + 31) & ~31) % nt;
+  const int npair = m / 2, nblk = npair * (npair - 1) / 2;
+  // this thread's first 2 x 2 block (planes P and P + k) and the steps to its next; the
+  // columns of V start at the warps after the last one with a block
+  const int P0 = tid % npair, k0 = 1 + tid / npair, dP = nt % npair, dk = nt / npair;
+  const int busy = ((nblk + 31) & ~31) % nt;
   const int v0 = tid >= busy ? tid - busy : tid + nt - busy;
   const int i0 = v0 % n, W0 = v0 / n, dI = nt % n, dW = nt / n;
   for (int sweep = 0; sweep < max_sweeps; sweep++) {
@@ -155,65 +169,60 @@ __device__ void jacobi_sweeps(R* A, R* V, int ld, int n, int m, Planes<R>& sh, R
         b += 1 + (b < 0 ? m - 1 : 0);
         const int p = min(a, b), q = max(a, b);
         const R app = A[tri(p, p)], aqq = A[tri(q, q)], apq = A[tri(q, p)];
-        R c, s;
+        float tan;
         if constexpr (k32) {
-          rotation32((aqq - app) + (sh.low[q] - sh.low[p]), apq, c, s);
-          if (fine && fabsf(s) > 1e-3f && fabsf(apq) > 1e-16f) sh.turned = 1;
+          const float h = half_tangent((aqq - app) + (sh.low[q] - sh.low[p]), apq, tan);
+          sh.h[tid] = h;
+          sh.s[tid] = sine(h);
+          sh.tan[tid] = tan;
+          if (fine && fabsf(tan) > 1e-3f && fabsf(apq) > 1e-16f) sh.turned = 1;
         } else {
-          rotation64(app, aqq, apq, c, s);
+          const float hf = half_tangent(d2f(aqq - app), d2f(apq), tan);
+          const double h = f2d(hf);
+          sh.h[tid] = h;
+          sh.s[tid] = sine(h, hf);
         }
-        sh.c[tid] = c;
-        sh.s[tid] = s;
         sh.p[tid] = p;
         sh.q[tid] = q;
       }
       __syncthreads();
       if (nt - 1 - tid < npair) {  // the planes' own diagonal blocks
         const int P = nt - 1 - tid;
-        const R c = sh.c[P], s = sh.s[P];
+        const R h = sh.h[P], s = sh.s[P];
         if (s != R(0)) {
           const int p = sh.p[P], q = sh.q[P];
           if constexpr (k32) {
             // app - t apq and aqq + t apq as two floats; the element between them is gone
-            const float x = __fdividef(s, c) * A[tri(q, p)];
+            const float x = sh.tan[P] * A[tri(q, p)];
             A[tri(q, p)] = 0.0f;
             add_low(A[tri(p, p)], sh.low[p], -x);
             add_low(A[tri(q, q)], sh.low[q], x);
           } else {
-            const R a = A[tri(p, p)], b = A[tri(q, p)], d = A[tri(q, q)];
-            const R x = c * a - s * b, y = c * b - s * d, z = s * a + c * b, w = s * b + c * d;
-            A[tri(p, p)] = c * x - s * y;
-            A[tri(q, p)] = s * x + c * y;
-            A[tri(q, q)] = s * z + c * w;
+            // as updates: their rounding scales with the angle, not with the diagonal
+            const R b = A[tri(q, p)], d = A[tri(p, p)] - A[tri(q, q)];
+            const R cs = fma(-h, s, R(1)) * s, ss = s * s, x = fma(ss, d, R(2) * cs * b);
+            A[tri(q, p)] = fma(cs, d, fma(R(-2) * ss, b, b));
+            A[tri(p, p)] -= x;
+            A[tri(q, q)] += x;
           }
         }
       }
-      // the 2 x 2 blocks of planes P and P + k (mod npair), each pair of planes once; a
-      // lane holds the block's row `row` and has the other from its neighbour
-      for (int e = tid, P = P0, k = k0; e - lane < nrow; e += nt) {
-        const bool in = e < nrow;
+      // the 2 x 2 blocks of planes P and Q = P + k (mod npair), each pair of planes once
+      for (int e = tid, P = P0, k = k0; e < nblk; e += nt) {
         const int Q = P + k < npair ? P + k : P + k - npair;
-        R own0 = R(0), own1 = R(0), cp = R(1), sp = R(0), cq = R(1), sq = R(0);
-        int at0 = 0, at1 = 0;
-        if (in) {
-          cp = sh.c[P];
-          sp = sh.s[P];
-          cq = sh.c[Q];
-          sq = sh.s[Q];
-          const int p = row ? sh.q[P] : sh.p[P];
-          at0 = tri(p, sh.p[Q]);
-          at1 = tri(p, sh.q[Q]);
-          own0 = A[at0];
-          own1 = A[at1];
-        }
-        if (__any_sync(kAll, sp != R(0) || sq != R(0))) {
-          const R oth0 = __shfl_xor_sync(kAll, own0, 1), oth1 = __shfl_xor_sync(kAll, own1, 1);
-          const R sr = row ? sp : -sp;
-          const R x = cp * own0 + sr * oth0, y = cp * own1 + sr * oth1;
-          if (in) {
-            A[at0] = cq * x - sq * y;
-            A[at1] = sq * x + cq * y;
-          }
+        const R hp = sh.h[P], sp = sh.s[P], hq = sh.h[Q], sq = sh.s[Q];
+        if (sp != R(0) || sq != R(0)) {
+          const int p = sh.p[P], q = sh.q[P], u = sh.p[Q], v = sh.q[Q];
+          const int pu = tri(p, u), pv = tri(p, v), qu = tri(q, u), qv = tri(q, v);
+          R a = A[pu], b = A[pv], c = A[qu], d = A[qv];
+          rotate(hp, sp, a, c);
+          rotate(hp, sp, b, d);
+          rotate(hq, sq, a, b);
+          rotate(hq, sq, c, d);
+          A[pu] = a;
+          A[pv] = b;
+          A[qu] = c;
+          A[qv] = d;
         }
         P += dP;
         k += dk;
@@ -223,13 +232,14 @@ __device__ void jacobi_sweeps(R* A, R* V, int ld, int n, int m, Planes<R>& sh, R
         }
       }
       for (int i = i0, P = W0; P < npair;) {
-        const R c = sh.c[P], s = sh.s[P];
+        const R h = sh.h[P], s = sh.s[P];
         if (s != R(0)) {
           R* vp = V + ld * sh.p[P] + i;
           R* vq = V + ld * sh.q[P] + i;
-          const R x = *vp, y = *vq;
-          *vp = c * x - s * y;
-          *vq = s * x + c * y;
+          R x = *vp, y = *vq;
+          rotate(h, s, x, y);
+          *vp = x;
+          *vq = y;
         }
         i += dI;
         P += dW;
@@ -402,17 +412,46 @@ __device__ __forceinline__ int ascending_rank(const double* A, int n, int j) {
 // Eigenvalues ascending at base + offE, eigenvectors in descending order at base + offU,
 // each with the sign that makes its largest-magnitude entry (the first one on ties)
 // positive -- the layout launch_reverse_columns produces. A is diagonal, times `scale`.
+// Equal eigenvalues (the zeros of a sector with empty blocks) keep the order that a selection
+// sort with exchanges leaves them in, since a cut may fall among them.
 __device__ void write_descending(const EigJob& jb, double* base, const double* A, const double* V, double scale,
                                  int* order) {
   const int n = jb.n, tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
-  for (int j = tid; j < n; j += blockDim.x) {
-    const int rk = ascending_rank(A, n, j);
-    base[jb.offE + rk] = A[tri(j, j)] / scale;
-    order[n - 1 - rk] = j;
+  if (tid < 32) {
+    for (int i = lane; i < n; i += 32) order[i] = i;
+    __syncwarp();
+    for (int i = 0; i < n; i++) {
+      double best = 0.0;
+      int at = n;
+      for (int j = i + lane; j < n; j += 32) {
+        const double v = A[tri(order[j], order[j])];
+        if (at == n || v < best) {
+          best = v;
+          at = j;
+        }
+      }
+      for (int d = 16; d > 0; d >>= 1) {
+        const double b2 = __shfl_xor_sync(0xffffffffu, best, d);
+        const int a2 = __shfl_xor_sync(0xffffffffu, at, d);
+        if (a2 < n && (at == n || b2 < best || (b2 == best && a2 < at))) {
+          best = b2;
+          at = a2;
+        }
+      }
+      at = __shfl_sync(0xffffffffu, at, 0);  // (lanes may differ on a NaN)
+      __syncwarp();
+      if (lane == 0) {
+        const int t = order[i];
+        order[i] = order[at];
+        order[at] = t;
+      }
+      __syncwarp();
+    }
   }
   __syncthreads();
+  for (int j = tid; j < n; j += blockDim.x) base[jb.offE + j] = A[tri(order[j], order[j])] / scale;
   for (int o = tid >> 5; o < n; o += nw) {
-    const double* col = V + v_ld(n) * order[o];
+    const double* col = V + v_ld(n) * order[n - 1 - o];
     double best = -1.0, v = 0.0;
     int at = n;
     for (int i = lane; i < n; i += 32)
@@ -483,10 +522,13 @@ __global__ void __launch_bounds__(kRrThreads, 1) rr_eig_kernel(const double* __r
   }
 }
 
-// The Gram matrices of the truncation: one CTA each; A, V and W as in eigen().
-__device__ __forceinline__ void gram_eigen(const EigJob& jb, double* base, double* A, double* V, double* W,
-                                           Planes<float>& shf, Planes<double>& sh, int* order) {
-  const int n = jb.n, m = even_up(n), tid = threadIdx.x, nt = blockDim.x;
+// The Gram matrices of the truncation, one CTA each, by FP64 sweeps throughout: a sector may
+// have to keep singular values far below 1e-8 of the largest, whose vectors the sweeps find
+// from the matrix's own small elements (which carry their own relative accuracy), while
+// V^T G V would round them to 1e-16 of the norm.
+__device__ __forceinline__ void gram_eigen(const EigJob& jb, double* base, double* A, double* V, Planes<double>& sh,
+                                           int* order) {
+  const int n = jb.n, m = even_up(n), ld = v_ld(n), tid = threadIdx.x, nt = blockDim.x;
   const double* G = base + jb.offG;
   double big = 0.0;
   for (int e = tid; e < n * n; e += nt) big = fmax(big, fabs(G[e]));
@@ -494,31 +536,25 @@ __device__ __forceinline__ void gram_eigen(const EigJob& jb, double* base, doubl
   for (int e = tid; e < m * m; e += nt) {
     const int i = e % m, j = e / m;
     if (j <= i) A[tri(i, j)] = i < n ? hs * G[i + n * j] + hs * G[j + n * i] : 0.0;
+    if (i < n) V[i + ld * j] = i == j ? 1.0 : 0.0;
   }
   __syncthreads();
-  if (n > 1) {
-    eigen(n, m, true, G, sc, A, V, W, shf, sh);
-  } else {
-    if (tid == 0) V[0] = 1.0;
-    __syncthreads();
-  }
+  if (n > 1) jacobi_sweeps<double>(A, V, ld, n, m, sh, 1e-30, 30);
   write_descending(jb, base, A, V, sc, order);
 }
 
 // order <= kBatchedEigMax
 constexpr int kEigSmallThreads = 512;
 __global__ void __launch_bounds__(kEigSmallThreads, 1) batched_eig_kernel(const EigJob* __restrict__ jobs,
-                                                                       double* __restrict__ base) {
+                                                                          double* __restrict__ base) {
   constexpr int kN = kBatchedEigMax;
-  __shared__ double A[tri_size(kN)], V[kN * v_ld(kN)], W[kN * kN];
+  __shared__ double A[tri_size(kN)], V[kN * v_ld(kN)];
   __shared__ Planes<double> sh;
-  __shared__ Planes<float> shf;
   __shared__ int order[kN];
-  gram_eigen(jobs[blockIdx.x], base, A, V, W, shf, sh, order);
+  gram_eigen(jobs[blockIdx.x], base, A, V, sh, order);
 }
 
-// order kBatchedEigMax + 1 .. kBatchedEigLargeMax: A and V in dynamic shared memory, the
-// eigenvectors' slot at offU as W until they are written there
+// order kBatchedEigMax + 1 .. kBatchedEigLargeMax: A and V in dynamic shared memory
 constexpr int kEigLargeThreads = 512;
 __host__ __device__ constexpr size_t eig_large_bytes(int n) {
   return sizeof(double) * (static_cast<size_t>(tri_size(even_up(n))) + static_cast<size_t>(even_up(n)) * v_ld(n));
@@ -527,10 +563,9 @@ __global__ void __launch_bounds__(kEigLargeThreads) batched_eig_large_kernel(con
                                                                              double* __restrict__ base) {
   extern __shared__ double dyn[];
   __shared__ Planes<double> sh;
-  __shared__ Planes<float> shf;
   __shared__ int order[kBatchedEigLargeMax];
   const EigJob jb = jobs[blockIdx.x];
-  gram_eigen(jb, base, dyn, dyn + tri_size(even_up(jb.n)), base + jb.offU, shf, sh, order);
+  gram_eigen(jb, base, dyn, dyn + tri_size(even_up(jb.n)), sh, order);
 }
 
 // Loewdin orthonormaliser of k <= 4 vectors: L = S^-1/2 from the k x k overlap S
