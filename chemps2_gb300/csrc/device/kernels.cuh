@@ -3,7 +3,8 @@
 //   block sandwich     every term out += alpha sum_p ratio_p op(A_p) op(B) op(C_p) of a
 //                      task-program stage, by output tiles, in three variants: the team
 //                      kernel for tiles up to 16 x 16 (sandwich_warp.cuh), the two-pass GEMM path for large groups
-//                      (intermediates once, then split-K item sums; sandwich_gemm.cu)
+//                      (intermediates once, then split-K item sums; sandwich_gemm.cu,
+//                      in FP64 also sandwich_digits.cu on the tensor cores)
 //                      and, for comparison only, the one-pass cooperative and
 //                      item-parallel kernels. Item sums run in a fixed order and split
 //                      tiles are reduced in split order, so results are deterministic.
@@ -134,6 +135,14 @@ cudaError_t launch_inter_tc(const InterJob* jobs, const GemmTile* tiles, int nti
 cudaError_t launch_sum_tc(const SumGroup* groups, const SumItem* items, const GemmTile* tiles, int ntiles,
                           double* partials, unsigned int* counters, const SlotPtrs& sp, unsigned int* sched, int* err,
                           cudaStream_t stream);
+
+// The two passes in FP64 on the tensor cores, as exact products of digits
+// (sandwich_digits.cu); `sched` and `err` as above.
+cudaError_t launch_inter_digits(const InterJob* jobs, const GemmTile* tiles, int ntiles, const SlotPtrs& sp,
+                                unsigned int* sched, int* err, cudaStream_t stream);
+cudaError_t launch_sum_digits(const SumGroup* groups, const SumItem* items, const GemmTile* tiles, int ntiles,
+                              double* partials, unsigned int* counters, const SlotPtrs& sp, unsigned int* sched,
+                              int* err, cudaStream_t stream);
 
 cudaError_t launch_sandwich(const Group* groups, const Term* terms, const BatchEntry* entries, const TileDesc* tiles,
                             int ntiles, const SlotPtrs& sp, cudaStream_t stream, Precision prec = Precision::kFP64);

@@ -1,0 +1,760 @@
+// Two-pass path of large groups in FP64 on the 5th-generation tensor cores: the passes of
+// sandwich_gemm.cu with every product of two FP64 blocks formed from exact integer products
+// of their digits (the splitting of K. Ozaki, T. Ogita, S. Oishi and S. Rump, "Error-free
+// transformations of matrix multiplication", 2012).
+//
+// Why: an SM of this GPU does 1.6 FP64 multiply-adds a clock and the tensor cores 4096
+// 16-bit ones, and sandwich_gemm.cu runs at the FP64 pipe's rate.
+//
+// A step is one product L (m x K) R (K x n) of at most 64 x 32 outputs and K <= 32. Each row
+// of L and column of R is scaled by the power of two above its largest magnitude, 2^e, and
+// every element becomes the integer X = v 2^(55 - e) to the nearest, |X| <= 2^55: seven
+// digits to the base 256, the first in [-128, 128], the others in [-128, 127], so exact in
+// FP16. (One scale for a whole block would do for norms, but not for the small rows and columns
+// of a vector graded by its singular values: their errors came out up to three times the FP64
+// pipe's.) The tensor core sums d_i d_j over K and over the pairs of one diagonal c = i + j <= 7
+// in FP32: at most 7 x 64 products of at most 2^14, below 2^24, so every sum is exact. Dropped
+// are the diagonals c >= 8, about 2^-64 of the largest product. The eight sums are put
+// together in 64-bit integers and rounded to a double by integer instructions; one FP64
+// instruction adds that to the item sum, where the FP64 pipe rounds at each of the K terms.
+// Products longer than 32 take several steps; a second one adds to the first one's sums in
+// tensor memory where its elements fit the same scales, and else to its rounded ones.
+// Measured against extended precision, random operands of one size or spread over 2^20: pass
+// 1 0.4 to 1.0e-16 of the norm (FP64 pipe 1.0 to 2.6e-16), pass 2 with 200 items 2.0 to 5.9e-16
+// (one rounding of each FP64-summed item: 2.9 to 7.8e-16).
+//
+// L's digits are rows of shared memory digit by digit and so are R's columns, so that digit i
+// of L meets digits 0 .. 7 - i of R in one MMA whose accumulator starts at column group i
+// (an eighth digit of R, of zeros, sets the last diagonal): 7 MMAs of M = 128 for each 16 of
+// K. Persistent 256-thread CTAs, two per SM (256 columns of tensor memory each, and 87 KB of
+// shared memory in pass 1, 104 in pass 2, so that one cuts digits and rounds sums while the
+// other's MMAs run) take the 64 x 32 halves of the tile lists' tiles from an atomic counter.
+// While the MMAs of a step run, all threads round the previous step's sums (copied from
+// tensor memory to shared memory by the warps of the quadrants that hold them) and the next
+// step's operands are on their way from memory. An operand that the step before had too is
+// not cut again.
+//
+// What bounds it: a step's fixed chain, load - exponents - digits - MMA - collect, of 2.1 to
+// 4 us an SM whatever its size, with the tensor pipe busy a fifth to a quarter of the time and
+// the issue slots 35 to 40 %. us a product and SM, FP64 pipe -> digits, pass 1 / pass 2:
+// 17 x 17 x 17 3.1 -> 2.4 / 4.2 -> 3.3, 32 x 32 x 32 8.3 -> 3.0 / 10.0 -> 4.3, 47 x 47 x 47 27 -> 9.0 /
+// 31 -> 10.6, 64 x 64 x 64 65 -> 12.2 / 73 -> 13.7. Below about 17 x 17 x 12 the FP64 pipe is the
+// faster one (digits_pay in runtime.cpp).
+//
+// Every mbarrier wait is bounded: after kTcSpinLimit polls the kernel records an error in
+// the runtime's mapped error word, frees its tensor memory and returns without writing its
+// tile. An infinite or NaN element makes its row's or column's outputs NaN; elements below the
+// normal range count as zero.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <cstddef>
+
+#include "kernels.cuh"
+#include "slots.cuh"
+#include "tcgen05.cuh"
+
+namespace c2g {
+
+namespace {
+
+constexpr int kDgThreads = 256;
+constexpr int kDgIssuer = 5;  // the warp that issues the MMAs: of the last to cut digits, and
+                              // without tile rows of tensor memory in a tile of 32 rows
+constexpr int kDgCtasPerSm = 2;
+constexpr int kDgDigits = 7, kDgDiagonals = 8;
+constexpr int kDgRows = 64, kDgCols = 32, kDgK = 32;  // of a step
+constexpr uint32_t kDgTmemCols = kDgDiagonals * kDgCols;
+constexpr int kDgBatch = 32;                          // records held in shared memory
+
+// K-major rows without swizzle, 16 of K at a time: 8-row groups of 256 bytes, 128 bytes
+// between the two 8-wide halves of K
+constexpr int kDgRowBytes = 32;
+constexpr int kDgLBytes = kDgDigits * kDgRows * kDgRowBytes;  // one half (16) of a step's K
+constexpr int kDgRBytes = (kDgDigits + 1) * kDgCols * kDgRowBytes;  // with a digit of zeros
+// leading dimension of a row of sums: 16-byte accesses of eight rows meet every bank once
+constexpr int kDgSumLd = kDgCols + 4;
+
+// One product: op(L) (rows x K) op(R) (K x cols), already at its tile.
+struct DgRecord {  // 64 bytes
+  const double* l;
+  const double* r;
+  double* s;  // pass 1: where it goes, column-major with leading dimension lds
+  double alpha;
+  int32_t lld, rld;  // element (i, k) of an operand: trans ? p[k + ld i] : p[i + ld k]
+  int32_t k, lds;
+  int16_t rows, cols;
+  int8_t ltrans, rtrans;
+  int8_t pad[10];
+};
+static_assert(sizeof(DgRecord) == 64, "DgRecord");
+
+struct __align__(1024) DgSmem {
+  unsigned char l[2 * kDgLBytes];
+  unsigned char r[2 * kDgRBytes];
+  int sums[kDgDiagonals / 2 * kDgRows * kDgSumLd];  // [diagonal pair][row][column] of the previous step
+  DgRecord rec[kDgBatch];
+  unsigned long long bar;
+  // largest exponent fields of the rows of L, then of the columns of R: of the step in
+  // flight, the one being staged and (zero) the next
+  alignas(16) unsigned int expo[3][kDgRows + kDgCols];
+  uint32_t tmem_base;
+  int slot, is_last;
+  // pass 2: a product's sums over its first steps, each thread's own outputs
+  double part[8][kDgThreads];
+};
+
+static_assert(offsetof(DgSmem, expo) % 16 == 0 && (kDgRows + kDgCols) % 4 == 0, "16-byte reads of expo");
+
+// Instruction descriptor of kind::f16: D F32 (bits 4-5 = 1), A and B F16 (bits 7-9 and 10-12
+// = 0), both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28; M = 128.
+__host__ __device__ constexpr uint32_t dg_idesc(int n) {
+  return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// Eight consecutive k of one row of an operand, in registers.
+struct DgUnit {
+  double v[8];
+};
+
+__device__ __forceinline__ void dg_load(DgUnit& u, const double* p, int ld, bool t, int row, int k0, int n) {
+  p += t ? k0 + static_cast<int64_t>(ld) * row : row + static_cast<int64_t>(ld) * k0;
+  const int64_t step = t ? 1 : ld;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    u.v[k] = k < n ? *p : 0.0;
+    p += step;
+  }
+}
+
+__device__ __forceinline__ unsigned int dg_exponent(const DgUnit& u) {
+  unsigned int e = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) e = max(e, static_cast<unsigned int>(__double2hiint(u.v[k])) & 0x7ff00000u);
+  return e >> 20;
+}
+
+// X + sum_i 128 256^i of an element: its digits less their sign, as bytes (the first digit as
+// nine bits); emax: the row's largest exponent field
+__device__ __forceinline__ unsigned long long dg_fixed(double v, unsigned int emax) {
+  const unsigned int hi = __double2hiint(v), lo = __double2loint(v);
+  const unsigned int e = (hi >> 20) & 0x7ffu;
+  const unsigned long long m =
+      (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 3;  // below 2^56
+  const unsigned int sh = e == 0u ? 63u : min(emax - e, 63u);
+  const unsigned long long x = ((m >> sh) + 1ull) >> 1;  // to the nearest, below 2^55
+  const unsigned long long s = static_cast<long long>(static_cast<int>(hi)) >> 63;
+  return (x ^ s) - s + 0x0080808080808080ull;
+}
+
+// digit i of two such integers as FP16, low first: 1024 + byte in FP16, less 1152
+template <int i>
+__device__ __forceinline__ uint32_t dg_pair(unsigned long long a, unsigned long long b) {
+  constexpr int byte = (6 - i) & 3;
+  const uint32_t x = static_cast<uint32_t>(i < 3 ? a >> 32 : a), y = static_cast<uint32_t>(i < 3 ? b >> 32 : b);
+  const uint32_t t = i == 0 ? __byte_perm(x, y, 0x7632) | 0x64006400u
+                            : (__byte_perm(x, y, byte | (4 + byte) << 8) & 0x00ff00ffu) | 0x64006400u;
+  const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&t), __floats2half2_rn(1152.0f, 1152.0f));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// Stores the digits of a unit (row `row`, k group kg of 8) of an operand; kRows: the rows of
+// a digit, half_bytes: the size of one half of K.
+template <int kRows>
+__device__ __forceinline__ void dg_store(const DgUnit& u, unsigned int emax, unsigned char* buf, int half_bytes,
+                                         int row, int kg) {
+  unsigned long long x[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) x[k] = dg_fixed(u.v[k], emax);
+  unsigned char* at = buf + (kg >> 1) * half_bytes + (kg & 1) * 128 + (row >> 3) * 256 + (row & 7) * 16;
+#define C2G_DIGIT(i)                                                                                       \
+  *reinterpret_cast<uint4*>(at + i * kRows * kDgRowBytes) =                                                \
+      make_uint4(dg_pair<i>(x[0], x[1]), dg_pair<i>(x[2], x[3]), dg_pair<i>(x[4], x[5]), dg_pair<i>(x[6], x[7]));
+  C2G_DIGIT(0)
+  C2G_DIGIT(1)
+  C2G_DIGIT(2)
+  C2G_DIGIT(3)
+  C2G_DIGIT(4)
+  C2G_DIGIT(5)
+  C2G_DIGIT(6)
+#undef C2G_DIGIT
+}
+
+// n 2^k as a double to the nearest, by the bits (a conversion or an FP64 instruction costs a
+// warp 65 clocks): zero where the result is below the normal range, infinite above it.
+__device__ __forceinline__ double rounded(long long n, int k) {
+  const unsigned long long s = static_cast<unsigned long long>(n >> 63);
+  unsigned long long u = (static_cast<unsigned long long>(n) ^ s) - s;
+  const int z = __clzll(static_cast<long long>(u));
+  u <<= z & 63;
+  const unsigned int hs = static_cast<unsigned int>(s) & 0x80000000u;
+  const int f = 1086 - z + k;  // the exponent field
+  if (u == 0ull || f <= 0) return __hiloint2double(hs, 0);
+  if (f >= 0x7fe) return __hiloint2double(hs | 0x7ff00000u, 0);
+  const unsigned long long m = (u + 0x400ull < u) ? 1ull << 53 : (u + 0x400ull) >> 11;  // 2^52 .. 2^53
+  const unsigned long long v = (static_cast<unsigned long long>(f - 1) << 52) + m;
+  return __hiloint2double(hs | static_cast<unsigned int>(v >> 32), static_cast<unsigned int>(v));
+}
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok));
+  return ok != 0;
+}
+
+// 16 accumulator columns of this thread's lane, not yet waited for
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+// (the registers pass through the wait, so no use of them moves before it)
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                 "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15])
+               :
+               : "memory");
+}
+
+// The running state of a CTA: the step in flight on the tensor cores and the sums so far.
+struct DgEngine {
+  DgSmem& sm;
+  uint32_t tmem;
+  uint32_t phase = 0u;
+  bool flying = false, ok = true;
+  int held = 0, cur = 1;  // exponent tables of the step in flight and of the one being staged
+  double alpha = 0.0;     // pass 2: of the step in flight
+  // the sums so far: row, columns col .. col + outputs - 1
+  double acc[8];
+
+  __device__ __forceinline__ DgEngine(DgSmem& s) : sm(s), tmem(s.tmem_base) { clear(); }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int k = 0; k < 8; k++) acc[k] = 0.0;
+  }
+  // A tile of up to 32 rows: 32 rows x 8 groups of 4 columns; of up to 64: 64 x 4 groups of 8.
+  __device__ __forceinline__ static int row_of(bool big) { return threadIdx.x & (big ? 63 : 31); }
+  __device__ __forceinline__ static int col_of(bool big) {
+    return big ? (threadIdx.x >> 6) * 8 : (threadIdx.x >> 5) * 4;
+  }
+
+  // Issues the MMAs of the staged step of 16 `halves` of K (one thread), `onto` the sums there. Digit i of L meets
+  // digits 0 .. 7 - i of R, the eighth of which is zero: it sets the last diagonal's sums.
+  __device__ __forceinline__ void issue(int halves, bool onto) {
+    tc_fence_after();
+    const uint64_t a0 = smem_desc(smem_u32(sm.l), 128, 256), b0 = smem_desc(smem_u32(sm.r), 128, 256);
+    for (int h = 0; h < halves; h++) {
+      const uint64_t a = a0 + static_cast<uint64_t>(h * (kDgLBytes >> 4));
+      const uint64_t b = b0 + static_cast<uint64_t>(h * (kDgRBytes >> 4));
+#pragma unroll
+      for (int i = 0; i < kDgDigits; i++)
+        tc_mma(tmem + i * kDgCols, a + static_cast<uint64_t>((i * kDgRows * kDgRowBytes) >> 4), b,
+               dg_idesc((kDgDiagonals - i) * kDgCols), (h == 0 && i == 0 && !onto) ? 0u : 1u);
+    }
+    tc_commit(&sm.bar);
+  }
+
+  __device__ __forceinline__ void wait() {
+    if (!mbar_wait(&sm.bar, phase)) ok = false;
+    phase ^= 1u;
+    tc_fence_after();
+  }
+
+  // Tensor memory -> shared memory: warp w holds rows 32 (w % 4) .. + 31 and columns
+  // 16 (w / 4) .. + 15. Two diagonals make one integer, 256 i_c + i_(c+1), below 2^30.
+  __device__ __forceinline__ void collect(int rows, int cols) {
+    const int warp = threadIdx.x >> 5, quad = warp & 3, c0 = 16 * (warp >> 2);
+    if (quad * 32 < rows && c0 < cols) {
+      const uint32_t from = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(c0);
+      int* to = sm.sums + (quad * 32 + (threadIdx.x & 31)) * kDgSumLd + c0;
+#pragma unroll
+      for (int c = 0; c < kDgDiagonals / 2; c++) {
+        uint32_t a[16], b[16];
+        tmem_ld16_async(from + 2 * c * kDgCols, a);
+        tmem_ld16_async(from + (2 * c + 1) * kDgCols, b);
+        tmem_wait_ld(a);
+        tmem_wait_ld(b);
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          int v[4];
+#pragma unroll
+          for (int t = 0; t < 4; t++)
+            v[t] = __float2int_rn(__uint_as_float(a[j + t])) * 256 + __float2int_rn(__uint_as_float(b[j + t]));
+          *reinterpret_cast<int4*>(to + c * kDgRows * kDgSumLd + j) = make_int4(v[0], v[1], v[2], v[3]);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+
+  // The collected sums, each rounded once: into acc (kSet), onto it (kAdd), or (kScale) with
+  // those of the product's other steps, times alpha, onto it: an item is rounded into acc
+  // once whatever its inner dimension, as on the FP64 pipe. An infinite or NaN element makes its row's or column's outputs NaN.
+  enum Mode { kSet, kAdd, kScale };
+  template <int kOut, Mode kMode>
+  __device__ __forceinline__ void finish(int rows, int cols, bool first, bool last) {
+    constexpr bool big = kOut == 8;
+    const int r = row_of(big), c0 = col_of(big);
+    if (r >= rows || c0 >= cols) return;
+    const int* s = sm.sums + r * kDgSumLd + c0;
+    const unsigned int* expo = sm.expo[held];
+    const unsigned int el = expo[r];
+#pragma unroll
+    for (int q = 0; q < kOut; q += 4) {
+      int p[4][4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const int4 t = *reinterpret_cast<const int4*>(s + c * kDgRows * kDgSumLd + q);
+        p[0][c] = t.x;
+        p[1][c] = t.y;
+        p[2][c] = t.z;
+        p[3][c] = t.w;
+      }
+      const uint4 e4 = *reinterpret_cast<const uint4*>(expo + kDgRows + c0 + q);
+      const unsigned int er[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int k = q + t;
+        // p0 2^-8 + p1 2^-24 + p2 2^-40 + p3 2^-56 to the nearest 2^-42, the size of the
+        // operands' own rounding; |p0| < 2^28 + 2^23, so below 2^63
+        const long long n = static_cast<long long>(p[t][0]) * (1ll << 34) + static_cast<long long>(p[t][1]) * (1 << 18) +
+                            static_cast<long long>(p[t][2]) * 4 + ((p[t][3] >> 14) + ((p[t][3] >> 13) & 1));
+        double v = rounded(n, static_cast<int>(el + er[t]) - 2044 - 56);
+        if (el == 0x7ffu || er[t] == 0x7ffu) v = __longlong_as_double(0x7ff8000000000000ll);
+        if constexpr (kMode == kScale) {
+          if (!first) v += sm.part[k][threadIdx.x];
+          if (last) acc[k] = fma(alpha, v, acc[k]);
+          else sm.part[k][threadIdx.x] = v;
+        } else if constexpr (kMode == kAdd) {
+          acc[k] += v;
+        } else {
+          acc[k] = v;
+        }
+      }
+    }
+  }
+  template <Mode kMode>
+  __device__ __forceinline__ void finish_any(int rows, int cols, bool first, bool last) {
+    if (rows > 32) finish<8, kMode>(rows, cols, first, last);
+    else finish<4, kMode>(rows, cols, first, last);
+  }
+};
+
+// Streams the products of sm.rec through the engine. Src: count(); prepare(q), called by all
+// threads before record q is read (it may refill sm.rec and hold barriers), returns its slot;
+// store(), called when a product's sums are complete (kEach: after every product; else the
+// sums of all products add up and stay in the engine).
+template <bool kEach, class Src>
+__device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
+  DgSmem& sm = E.sm;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  // The digits are cut first by the warps that hold no tile rows of tensor memory (those of
+  // quadrants 2 and 3), which need not copy sums meanwhile: warps 2, 3, 6, 7, 1, 5, 0, 4.
+  const int utid = static_cast<int>((0x32571046u >> (4 * warp)) & 0xfu) * 32 + lane;
+
+  int q = 0, k0 = 0, slot = 0;
+  bool more = false;
+  const int n = src.count();
+  auto seek = [&]() {  // the first product with an inner dimension at or after q
+    more = false;
+    for (; q < n; q++) {
+      slot = src.prepare(q);
+      if (sm.rec[slot].k > 0) {
+        k0 = 0;
+        more = true;
+        return;
+      }
+    }
+  };
+  // The step's units: rows of L, then rows of R, over its k groups; this thread's first and
+  // second. Packed: row | k group << 8 | (of L) << 12 | valid << 13.
+  DgUnit u0, u1;
+  int w0 = 0, w1 = 0;
+  bool same_l = false, same_r = false;  // the operand is that of the step before, already cut
+  auto fetch = [&](DgUnit& u, int e) -> int {
+    const DgRecord& X = sm.rec[slot];
+    const int rows = X.rows, cols = X.cols, rem = X.k - k0, kgc = rem > 16 ? 4 : 2;
+    const int lsh = rows > 32 ? 6 : 5, rsh = cols > 16 ? 5 : 4;
+    const int nl = same_l ? 0 : kgc << lsh, nr = same_r ? 0 : kgc << rsh;
+    if (e >= nl + nr) return 0;
+    const bool is_l = e < nl;
+    const int f = is_l ? e : e - nl, sh = is_l ? lsh : rsh, row = f & ((1 << sh) - 1), kg = f >> sh;
+    if (row >= (is_l ? rows : cols)) return is_l ? 1 << 12 : 0;
+    dg_load(u, is_l ? X.l : X.r, is_l ? X.lld : X.rld, is_l ? X.ltrans : X.rtrans, row, k0 + 8 * kg, rem - 8 * kg);
+    return row | kg << 8 | (is_l ? 1 << 12 : 0) | 1 << 13;
+  };
+  auto cut = [&](const DgUnit& u, int w, const unsigned int* expo) {
+    if (!(w & (1 << 13))) return;
+    const int row = w & 0xff, kg = (w >> 8) & 0xf;
+    if (w & (1 << 12)) dg_store<kDgRows>(u, expo[row], sm.l, kDgLBytes, row, kg);
+    else dg_store<kDgCols>(u, expo[kDgRows + row], sm.r, kDgRBytes, row, kg);
+  };
+
+  // the previous step's product: its extents, and in pass 1 where it goes and whether complete
+  int prows = 0, pcols = 0, plds = 0;
+  double* ps = nullptr;
+  bool pfirst = false, plast = false;
+  auto complete = [&]() {
+    if constexpr (kEach) {
+      if (pfirst) E.template finish_any<DgEngine::kSet>(prows, pcols, true, true);
+      else E.template finish_any<DgEngine::kAdd>(prows, pcols, true, true);
+      if (plast) src.store(E, ps, plds, prows, pcols);
+    } else {
+      E.template finish_any<DgEngine::kScale>(prows, pcols, pfirst, plast);
+    }
+  };
+
+  seek();
+  if (more) {
+    w0 = fetch(u0, utid);
+    w1 = fetch(u1, utid + kDgThreads);
+  }
+  while (more) {
+    unsigned int* expo = sm.expo[E.cur];
+    const unsigned int* before = sm.expo[E.held];
+    // the rows' and columns' largest exponents, or those already there
+    if (w0 & (1 << 13)) atomicMax(expo + (w0 & 0xff) + (w0 & (1 << 12) ? 0 : kDgRows), dg_exponent(u0));
+    if (w1 & (1 << 13)) atomicMax(expo + (w1 & 0xff) + (w1 & (1 << 12) ? 0 : kDgRows), dg_exponent(u1));
+    if (tid < kDgRows + kDgCols && (tid < kDgRows ? same_l : same_r)) expo[tid] = before[tid];
+    __syncthreads();
+    const int spare = 3 - E.held - E.cur;  // last read a step ago
+    if (tid < kDgRows + kDgCols) sm.expo[spare][tid] = 0u;
+    // The second 32 of K go onto the first ones' sums where their scales will do: the sums of
+    // 64 products of a diagonal are exact as well, and pairs of them below 2^31.
+    bool onto = false;
+    if (k0 == kDgK && E.flying) onto = !__syncthreads_or(tid < kDgRows + kDgCols && expo[tid] > before[tid]);
+    if (E.flying) {
+      E.wait();
+      if (!onto) E.collect(prows, pcols);
+    }
+    // the digits (the MMAs that read the buffers are done)
+    cut(u0, w0, onto ? before : expo);
+    cut(u1, w1, onto ? before : expo);
+    fence_async_smem();
+    if (__syncthreads_or(!E.ok)) return false;
+    const DgRecord& X = sm.rec[slot];
+    const int rem = X.k - k0;
+    if (warp == kDgIssuer) {
+      if (elect_one()) E.issue(rem > 16 ? 2 : 1, onto);
+      __syncwarp();
+    }
+    const double alpha = X.alpha;
+    const int rows = X.rows, cols = X.cols, lds = X.lds;
+    double* const s = X.s;
+    const bool first = k0 == 0, last = rem <= kDgK;
+    // the next step's operands; an operand that this step staged as well is not read again
+    same_l = same_r = false;
+    if (!last) {
+      k0 += kDgK;
+    } else {
+      const double *l = X.l, *r = X.r;
+      const int lld = X.lld, rld = X.rld, k = X.k, trans = X.ltrans | X.rtrans << 8;
+      q++;
+      seek();
+      if (more && first) {
+        const DgRecord& N = sm.rec[slot];
+        same_l = N.k == k && N.l == l && N.lld == lld && N.ltrans == (trans & 0xff) && N.rows == rows;
+        same_r = N.k == k && N.r == r && N.rld == rld && N.rtrans == trans >> 8 && N.cols == cols;
+      }
+    }
+    if (more) {
+      w0 = fetch(u0, utid);
+      w1 = fetch(u1, utid + kDgThreads);
+    }
+    if (E.flying && !onto) complete();
+    E.flying = true;
+    E.alpha = alpha;
+    if (!onto) E.held = E.cur;
+    E.cur = spare;
+    prows = rows;
+    pcols = cols;
+    plds = lds;
+    ps = s;
+    pfirst = first || (onto && pfirst);
+    plast = last;
+  }
+  if (E.flying) {
+    __syncthreads();  // the last sums have been read
+    E.wait();
+    E.collect(prows, pcols);
+    if (__syncthreads_or(!E.ok)) return false;
+    complete();
+    E.flying = false;
+  }
+  return true;
+}
+
+// Pass 1: a batch of job tiles, each in up to two column halves.
+struct DgInterSource {
+  int units;
+  __device__ __forceinline__ int count() const { return units; }
+  __device__ __forceinline__ int prepare(int q) const { return q; }
+  __device__ __forceinline__ void store(const DgEngine& E, double* s, int lds, int rows, int cols) const {
+    const bool big = rows > 32;
+    const int r = DgEngine::row_of(big), c0 = DgEngine::col_of(big);
+    if (r >= rows) return;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (k < (big ? 8 : 4) && c0 + k < cols) s[r + static_cast<int64_t>(lds) * (c0 + k)] = E.acc[k];
+  }
+};
+
+// Pass 2: the items of a tile half, their records made from the item list kDgBatch at a time.
+struct DgSumSource {
+  const SumItem* items;
+  int item0, item1;
+  const SlotPtrs& sp;
+  DgSmem& sm;
+  int row0, col0, rows, cols;
+  int held = -1;  // first item held (uniform)
+  __device__ __forceinline__ int count() const { return item1 - item0; }
+  __device__ __forceinline__ int prepare(int q) {
+    if (held < 0 || q >= held + kDgBatch) {  // q never goes back
+      __syncthreads();
+      const int n = min(kDgBatch, item1 - item0 - q);
+      if (static_cast<int>(threadIdx.x) < n) {
+        const SumItem I = items[item0 + q + threadIdx.x];
+        DgRecord d{};
+        d.k = I.k;
+        if (I.k > 0) {
+          d.l = resolve<double>(sp, I.l.ref) + (I.l.trans ? static_cast<int64_t>(I.l.ld) * row0 : row0);
+          d.r = resolve<double>(sp, I.r.ref) + (I.r.trans ? col0 : static_cast<int64_t>(I.r.ld) * col0);
+        }
+        d.lld = I.l.ld;
+        d.rld = I.r.ld;
+        d.ltrans = I.l.trans != 0;
+        d.rtrans = I.r.trans == 0;  // a row of R's digits is a column of op(R)
+        d.alpha = I.alpha;
+        d.rows = static_cast<int16_t>(rows);
+        d.cols = static_cast<int16_t>(cols);
+        sm.rec[threadIdx.x] = d;
+      }
+      held = q;
+      __syncthreads();
+    }
+    return q - held;
+  }
+};
+
+__device__ void dg_setup(DgSmem& sm) {
+  if (threadIdx.x == 0) {
+    mbar_init(&sm.bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int i = threadIdx.x; i < 3 * (kDgRows + kDgCols); i += kDgThreads)
+    sm.expo[i / (kDgRows + kDgCols)][i % (kDgRows + kDgCols)] = 0u;
+  // the digit of zeros of either half of R's K
+  constexpr int kZero = kDgCols * kDgRowBytes;
+  for (int i = threadIdx.x; i < 2 * kZero / 4; i += kDgThreads)
+    *reinterpret_cast<uint32_t*>(sm.r + (i / (kZero / 4)) * kDgRBytes + kDgDigits * kZero + 4 * (i % (kZero / 4))) = 0u;
+  fence_async_smem();
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
+                 "r"(kDgTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+}
+
+__device__ void dg_teardown(uint32_t tmem_d) {
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kDgTmemCols) : "memory");
+  }
+}
+
+// The next `take` of the work list.
+__device__ __forceinline__ int dg_next(unsigned int* sched, int* slot, int take) {
+  __syncthreads();  // the previous work's epilogue is done in every thread
+  if (threadIdx.x == 0) *slot = static_cast<int>(atomicAdd(sched, static_cast<unsigned int>(take)));
+  __syncthreads();
+  return *slot;
+}
+
+__device__ __forceinline__ void dg_end(DgEngine& E, unsigned int* sched, int* err) {
+  if (__syncthreads_or(!E.ok)) {
+    if (threadIdx.x == 0 && err) atomicOr(err, 2);
+    mbar_wait(&E.sm.bar, E.phase ^ 1u);  // the MMAs still in flight, bounded again
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(sched + 1, 1u) == gridDim.x - 1) {
+    sched[0] = 0u;
+    sched[1] = 0u;
+  }
+  dg_teardown(E.tmem);
+}
+
+// Pass 1, `take` job tiles at a time.
+__global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
+    inter_digits_kernel(const InterJob* __restrict__ jobs, const GemmTile* __restrict__ tiles, int ntiles, int take,
+                        SlotPtrs sp, unsigned int* sched, int* err) {
+  extern __shared__ unsigned char dyn[];
+  DgSmem& sm = *reinterpret_cast<DgSmem*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
+  dg_setup(sm);
+  DgEngine E(sm);
+  for (;;) {
+    const int first = dg_next(sched, &sm.slot, take);
+    if (first >= ntiles) break;
+    const int n = min(take, ntiles - first);
+    if (static_cast<int>(threadIdx.x) < 2 * n) {
+      const GemmTile T = tiles[first + (threadIdx.x >> 1)];
+      const InterJob J = jobs[T.idx];
+      const int row0 = (T.pos >> 16) * 64, col0 = (T.pos & 0xffff) * 64 + (threadIdx.x & 1) * kDgCols;
+      DgRecord d{};
+      d.rows = static_cast<int16_t>(min(64, J.m - row0));
+      d.cols = static_cast<int16_t>(min(kDgCols, J.n - col0));
+      d.k = d.cols > 0 ? J.k : 0;
+      if (d.cols > 0) {
+        d.l = resolve<double>(sp, J.l.ref) + (J.l.trans ? static_cast<int64_t>(J.l.ld) * row0 : row0);
+        d.r = resolve<double>(sp, J.r.ref) + (J.r.trans ? col0 : static_cast<int64_t>(J.r.ld) * col0);
+        d.s = sp.inter + J.off + row0 + static_cast<int64_t>(J.m) * col0;
+      }
+      d.alpha = 1.0;
+      d.lld = J.l.ld;
+      d.rld = J.r.ld;
+      d.lds = J.m;
+      d.ltrans = J.l.trans != 0;
+      d.rtrans = J.r.trans == 0;
+      sm.rec[threadIdx.x] = d;
+    }
+    __syncthreads();
+    DgInterSource src{2 * n};
+    if (!dg_stream<true>(E, src)) break;
+  }
+  dg_end(E, sched, err);
+}
+
+// Pass 2: the column halves of the tiles one after another; a tile at most 32 columns wide
+// has one.
+__global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
+    sum_digits_kernel(const SumGroup* __restrict__ groups, const SumItem* __restrict__ items,
+                      const GemmTile* __restrict__ tiles, int ntiles, double* partials, unsigned int* counters,
+                      SlotPtrs sp, unsigned int* sched, int* err) {
+  extern __shared__ unsigned char dyn[];
+  DgSmem& sm = *reinterpret_cast<DgSmem*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
+  dg_setup(sm);
+  DgEngine E(sm);
+  for (;;) {
+    const int t = dg_next(sched, &sm.slot, 1);
+    if (t >= 2 * ntiles) break;
+    const GemmTile T = tiles[t >> 1];
+    const SumGroup G = groups[T.idx];
+    const int row0 = (T.pos >> 16) * 64, tcol0 = (T.pos & 0xffff) * 64, off = (t & 1) * kDgCols, col0 = tcol0 + off;
+    const int tm = min(64, G.m - row0), tn = min(kDgCols, G.n - col0);
+    if (tn <= 0) continue;
+    E.clear();
+    DgSumSource src{items, T.item0, T.item1, sp, sm, row0, col0, tm, tn};
+    if (!dg_stream<false>(E, src)) break;
+    const bool big = tm > 32, mine = DgEngine::row_of(big) < tm;
+    const int r = DgEngine::row_of(big), c0 = DgEngine::col_of(big), nout = big ? 8 : 4;
+    // items without an inner dimension: out += alpha op(R)
+    if (mine)
+      for (int it = T.item0; it < T.item1; it++) {
+        const SumItem& I = items[it];
+        if (I.k > 0) continue;
+        const double* R = resolve<double>(sp, I.r.ref);
+        const int64_t si = I.r.trans ? I.r.ld : 1, sj = I.r.trans ? 1 : I.r.ld;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (k < nout && c0 + k < tn) E.acc[k] = fma(I.alpha, R[(row0 + r) * si + (col0 + c0 + k) * sj], E.acc[k]);
+      }
+    double* O = const_cast<double*>(resolve<double>(sp, G.out));
+    const int64_t ldo = G.ldo;
+    const bool accum = (G.flags & kAccumulate) != 0;
+    if (T.nsplit == 1) {
+      if (mine)
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (k < nout && c0 + k < tn) {
+            const int64_t idx = (row0 + r) + ldo * (col0 + c0 + k);
+            O[idx] = accum ? O[idx] + E.acc[k] : E.acc[k];
+          }
+      continue;
+    }
+    // a split tile: the last unit (split x column half) to arrive adds the splits in order
+    const int TM = 16 * ((T.shape & 3) + 1), TN = 16 * (((T.shape >> 2) & 3) + 1);
+    double* part = partials + T.part;
+    const int64_t te = static_cast<int64_t>(TM) * TN;
+    if (mine)
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k < nout && c0 + k < tn) __stcg(part + T.split * te + r + TM * (off + c0 + k), E.acc[k]);
+    const int width = min(64, G.n - tcol0);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+      sm.is_last = atomicAdd(counters + T.counter, 1u) ==
+                   static_cast<unsigned>(T.nsplit * ((width + kDgCols - 1) / kDgCols) - 1);
+    __syncthreads();
+    if (!sm.is_last) continue;
+    __threadfence();
+    if (threadIdx.x == 0) counters[T.counter] = 0u;  // ready for the next launch
+    for (int e = threadIdx.x; e < tm * width; e += kDgThreads) {
+      const int i = e % tm, c = e / tm;
+      double v = 0.0;
+      for (int s = 0; s < T.nsplit; s++) v += __ldcg(part + s * te + i + TM * c);
+      const int64_t idx = (row0 + i) + ldo * (tcol0 + c);
+      O[idx] = accum ? O[idx] + v : v;
+    }
+  }
+  dg_end(E, sched, err);
+}
+
+constexpr int kDgSmemBytes = static_cast<int>(sizeof(DgSmem)) + 1024;
+constexpr int kDgInterBytes = static_cast<int>(offsetof(DgSmem, part)) + 1024;  // what pass 1 uses of it
+
+int dg_grid(int units) {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 152;
+    return n;
+  }();
+  return std::min(units, kDgCtasPerSm * sms);
+}
+
+}  // namespace
+
+cudaError_t launch_inter_digits(const InterJob* jobs, const GemmTile* tiles, int ntiles, const SlotPtrs& sp,
+                                unsigned int* sched, int* err, cudaStream_t stream) {
+  if (ntiles <= 0) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(inter_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgInterBytes);
+  if (e != cudaSuccess) return e;
+  const int grid = dg_grid(ntiles);
+  // several batches a CTA, so that no CTA is left with a long one at the end
+  const int take = std::max(1, std::min(kDgBatch / 2, ntiles / (4 * grid)));
+  inter_digits_kernel<<<grid, kDgThreads, kDgInterBytes, stream>>>(jobs, tiles, ntiles, take, sp, sched, err);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sum_digits(const SumGroup* groups, const SumItem* items, const GemmTile* tiles, int ntiles,
+                              double* partials, unsigned int* counters, const SlotPtrs& sp, unsigned int* sched,
+                              int* err, cudaStream_t stream) {
+  if (ntiles <= 0) return cudaSuccess;
+  const cudaError_t e =
+      cudaFuncSetAttribute(sum_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
+  if (e != cudaSuccess) return e;
+  sum_digits_kernel<<<dg_grid(2 * ntiles), kDgThreads, kDgSmemBytes, stream>>>(groups, items, tiles, ntiles, partials,
+                                                                                counters, sp, sched, err);
+  return cudaGetLastError();
+}
+
+}  // namespace c2g

@@ -33,6 +33,23 @@ int warp_slots(int cls) {
   return 4 * 32 / (gr[warp_row_class(cls)] * gc[cls % kWarpColClasses]);
 }
 
+// Whether a tile of PM x PN units of 16 x 16 is formed from digits on the tensor cores
+// (sandwich_digits.cu) in FP64 runs; `k`: the inner dimension, summed over `products`
+// products. A digit step costs about the same (2.1 to 4.3 us of an SM) whatever its size up
+// to 64 x 32 x 32, the FP64 pipe 0.16 us (pass 1) to 0.2 us for each of PM PN k / 4: measured,
+// 32 x 32 tiles (17 x 17 to 32 x 32 blocks), us a product and SM: k = 8 1.7 against 2.1 (pass 1)
+// and 2.1 against 2.8 (pass 2), k = 17 3.1 against 2.4 and 4.2 against 3.3, 32 x 32 x 32 8.3
+// against 3.0 and 10.0 against 4.3, 64 x 64 x 64 65 against 12 and 73 against 14. So one tile
+// alone breaks even at PM PN k of about 45 for each column half of 32; whole matvecs, where
+// the tiles left to the FP64 pipe are few, do best with the line at 24 to 40 (L = 24 D2h
+// D = 1000 14.4, 13.8, 13.9, 14.1 ms at 0, 24, 40, 56; Hubbard L = 18 D = 400 10.1, 10.7, 10.7,
+// 10.8 ms, against 14.5 and 28.2 ms on the FP64 pipe alone).
+constexpr int64_t kDigitsLine = 32;
+bool digits_pay(int shape, int64_t k, int64_t products) {
+  const int pm = (shape & 3) + 1, pn = ((shape >> 2) & 3) + 1;
+  return pm * pn * k >= kDigitsLine * ((pn + 1) / 2) * products;
+}
+
 // The team variant spreads a stage over at least this many CTA-sized pieces of work, and
 // splits a tile over at most kWarpMaxSplit CTAs.
 constexpr int64_t kWarpCtaTarget = 2048;
@@ -890,6 +907,26 @@ std::unique_ptr<DevProgram> Runtime::upload_parts(const Program* parts, size_t n
             static_cast<int>(tp.small_first[q0]), static_cast<int>(tp.small_first[q1] - tp.small_first[q0]),
             static_cast<int>(stile_of[q0]), static_cast<int>(stile_of[q1] - stile_of[q0])};
       }
+      // within a chunk, the tiles that digits form first
+      std::vector<int64_t> ksum(tp.items.size() + 1, 0);
+      for (size_t i = 0; i < tp.items.size(); i++) ksum[i + 1] = ksum[i] + std::max(tp.items[i].k, 0);
+      for (DevStage::PassChunk& ch : chunk_ranges[s]) {
+        GemmTile* j0 = tp.jtiles.data() + ch.jtile0;
+        ch.njdigits = static_cast<int>(std::stable_partition(j0, j0 + ch.njtiles,
+                                                             [&](const GemmTile& t) {
+                                                               return digits_pay(t.shape, tp.jobs[t.idx].k, 1);
+                                                             }) -
+                                       j0);
+        GemmTile* s0 = tp.stiles.data() + ch.stile0;
+        // (by the group's items: all splits of a tile meet at one counter)
+        ch.nsdigits = static_cast<int>(std::stable_partition(s0, s0 + ch.nstiles,
+                                                             [&](const GemmTile& t) {
+                                                               const SumGroup& g = tp.groups[t.idx];
+                                                               return digits_pay(t.shape, ksum[g.i1] - ksum[g.i0],
+                                                                                 g.i1 - g.i0);
+                                                             }) -
+                                       s0);
+      }
       if (tp.items.size() > size_t(INT32_MAX) || tp.jobs.size() > size_t(INT32_MAX))
         throw std::length_error("upload: too many large-group items");
     }
@@ -1011,28 +1048,62 @@ void Runtime::launch_stage(const DevProgram& p, const DevStage& ds, const SlotPt
   unsigned* gemm_counters = transient_counters(kTransientGemmCounters, p.gemm_counter_count);
   double* partials = transient_doubles(kTransientPartials, p.part_size);
   unsigned* counters = transient_counters(kTransientCounters, p.counter_count);
-  int npass = 0;
+  // Kernels that do not depend on one another run on two streams, so that the first CTAs of
+  // one fill the SMs that the last ones of another leave idle: the two halves of either pass
+  // (digits and FP64 pipe), and the team variant beside the passes.
+  const WarpLaunch wl{ds.groups, ds.terms, p.entries, ds.tiles_warp, partials, counters};
+  bool team_due = ds.ntiles_warp > 0;
+  const bool two = !ds.chunks.empty() && (team_due || prec == Precision::kFP64);
+  cudaStream_t other = stream_;
+  if (two) {
+    fork_aux();
+    other = aux_stream();
+  }
+  auto team = [&] {
+    if (team_due) C2G_CUDA(launch_sandwich_warp(wl, ds.ntiles_warp, sp, other, prec));
+    team_due = false;
+  };
+  int nlaunch = ds.ntiles_warp > 0;
   for (const DevStage::PassChunk& ch : ds.chunks) {
     const GemmTile* jt = ds.jtiles + ch.jtile0;
-    if (prec_run == Precision::kTC)
-      C2G_CUDA(launch_inter_tc(ds.jobs, jt, ch.njtiles, sp, sched_, err_dev_, stream_));
-    else
-      C2G_CUDA(launch_inter_gemm(ds.jobs, jt, ch.njtiles, sp, stream_, prec));
-    C2G_CUDA(launch_inter_small(ds.jobs, ds.jsmall + ch.small0, ch.nsmall, sp, stream_, prec));
     const GemmTile* st = ds.stiles + ch.stile0;
-    if (prec_run == Precision::kTC)
+    if (prec_run == Precision::kTC) {
+      C2G_CUDA(launch_inter_tc(ds.jobs, jt, ch.njtiles, sp, sched_, err_dev_, stream_));
+      C2G_CUDA(launch_inter_small(ds.jobs, ds.jsmall + ch.small0, ch.nsmall, sp, stream_, prec));
+      team();
       C2G_CUDA(launch_sum_tc(ds.sgroups, ds.sitems, st, ch.nstiles, gemm_partials, gemm_counters, sp, sched_ + 2,
                              err_dev_, stream_));
-    else
-      C2G_CUDA(launch_sum_gemm(ds.sgroups, ds.sitems, st, ch.nstiles, gemm_partials, gemm_counters, sp, stream_,
-                               prec));
-    npass += (ch.njtiles > 0) + (ch.nsmall > 0) + (ch.nstiles > 0);
+      nlaunch += (ch.njtiles > 0) + (ch.nsmall > 0) + (ch.nstiles > 0);
+      continue;
+    }
+    const bool fp64 = prec == Precision::kFP64;
+    const int nj = fp64 ? ch.njdigits : 0, ns = fp64 ? ch.nsdigits : 0;
+    cudaStream_t side = fp64 ? other : stream_;
+    C2G_CUDA(launch_inter_digits(ds.jobs, jt, nj, sp, sched_, err_dev_, stream_));
+    C2G_CUDA(launch_inter_gemm(ds.jobs, jt + nj, ch.njtiles - nj, sp, side, prec));
+    C2G_CUDA(launch_inter_small(ds.jobs, ds.jsmall + ch.small0, ch.nsmall, sp, side, prec));
+    // pass 2 reads all of pass 1, on either stream
+    if (side != stream_) {
+      join_aux();
+      if (ns < ch.nstiles) fork_aux();
+    }
+    C2G_CUDA(launch_sum_digits(ds.sgroups, ds.sitems, st, ns, gemm_partials, gemm_counters, sp, sched_ + 2, err_dev_,
+                               stream_));
+    C2G_CUDA(launch_sum_gemm(ds.sgroups, ds.sitems, st + ns, ch.nstiles - ns, gemm_partials, gemm_counters, sp, side,
+                             prec));
+    team();
+    // the next chunk's pass 1 overwrites the intermediates that this pass 2 reads
+    if (side != stream_ && &ch != &ds.chunks.back()) {
+      join_aux();
+      fork_aux();
+    }
+    nlaunch += (nj > 0) + (nj < ch.njtiles) + (ch.nsmall > 0) + (ns > 0) + (ns < ch.nstiles);
   }
   C2G_CUDA(launch_sandwich_tiles(ds.groups, ds.terms, p.entries, ds.tiles_large, ds.ntiles_large, sp, stream_, prec));
-  const WarpLaunch wl{ds.groups, ds.terms, p.entries, ds.tiles_warp, partials, counters};
-  C2G_CUDA(launch_sandwich_warp(wl, ds.ntiles_warp, sp, stream_, prec));
+  team();
   C2G_CUDA(launch_sandwich(ds.groups, ds.terms, p.entries, ds.tiles, ds.ntiles, sp, stream_, prec));
-  count_launches(npass + (ds.ntiles > 0) + (ds.ntiles_large > 0) + (ds.ntiles_warp > 0));
+  if (two) join_aux();
+  count_launches(nlaunch + (ds.ntiles > 0) + (ds.ntiles_large > 0));
 }
 
 void Runtime::sync() {

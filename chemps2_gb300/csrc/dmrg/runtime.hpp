@@ -48,8 +48,11 @@ struct DevStage {
   // The large groups in chunks of whole groups, each run as pass 1 then pass 2, so that
   // the intermediates of one chunk at a time share the intermediate buffer: ranges of
   // jtiles, jsmall and stiles.
+  // Of a chunk's job tiles and pass-2 tiles, the first njdigits and nsdigits are those that
+  // FP64 runs form from digits on the tensor cores (digits_pay).
   struct PassChunk {
     int jtile0, njtiles, small0, nsmall, stile0, nstiles;
+    int njdigits = 0, nsdigits = 0;
   };
   std::vector<PassChunk> chunks;
   int64_t flops = 0, items = 0;
