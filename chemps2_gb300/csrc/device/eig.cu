@@ -26,7 +26,8 @@
 //     table below, but round small eigenvalues to 1e-16 of the norm.
 // Measured, 20 Gram matrices of Gaussian / graded (1 to 1e-18) spectrum, against FP64 sweeps
 // of four operations on the full matrix: order 16 0.48 / 0.85 -> 0.17 / 0.29 ms, 32 2.34 / 3.99
-// -> 0.53 / 0.92, 64 6.2 / 11.7 -> 2.9 / 5.6, 128 41 / 82 -> 21 / 47, with errors of the
+// -> 0.53 / 0.92, 64 6.2 / 11.7 -> 2.9 / 5.6, 128 41 / 82 -> 21 / 47 (one CTA for each; up to 38
+// matrices above order 32 take a cluster each, 1.1 to 4 times as fast), with errors of the
 // eigenvalues and the orthogonality of 0.3 to 2.6e-15 (2 to 70e-15 before). Rayleigh-Ritz
 // of order 16: 332 -> 121 us cold, 177 -> 92 us warm; 32: 982 -> 357 and 584 -> 269.
 #include "kernels.cuh"
@@ -109,6 +110,29 @@ __device__ __forceinline__ void add_low(float& hi, float& lo, float x) {
   hi = s;
 }
 
+// Pair t of round r of m players: pos(0) = 0, pos(k) = 1 + (k - 1 - r mod m - 1), and the
+// pairs are (pos(t), pos(m - 1 - t))
+__device__ __forceinline__ void round_pair(int t, int r, int m, int& p, int& q) {
+  int a = 0, b = m - 2 - t - r;
+  if (t > 0) {
+    a = t - 1 - r;
+    a += 1 + (a < 0 ? m - 1 : 0);
+  }
+  b += 1 + (b < 0 ? m - 1 : 0);
+  p = min(a, b);
+  q = max(a, b);
+}
+
+// A plane's own diagonal block, as updates: their rounding scales with the angle, not with
+// the diagonal
+__device__ __forceinline__ void turn_plane(double h, double s, double& app, double& aqp, double& aqq) {
+  const double b = aqp, d = app - aqq;
+  const double cs = fma(-h, s, 1.0) * s, ss = s * s, x = fma(ss, d, 2.0 * cs * b);
+  aqp = fma(cs, d, fma(-2.0 * ss, b, b));
+  app -= x;
+  aqq += x;
+}
+
 // Jacobi sweeps on the packed m x m matrix A (m even, entries of magnitude <= 1 or so; an
 // odd order is padded by a zero row), the rotations applied to the columns of V (rows
 // 0 .. n - 1, column j at V + ld j). FP64: until off(A)^2 <= tol |A|^2. FP32: until off(A)^2 is
@@ -160,14 +184,8 @@ __device__ void jacobi_sweeps(R* A, R* V, int ld, int n, int m, Planes<R>& sh, R
     if (tid == 0) sh.turned = 0;
     for (int r = 0; r < m - 1; r++) {
       if (tid < npair) {
-        // pos(0) = 0, pos(k) = 1 + (k - 1 - r mod m - 1); pairs (pos(t), pos(m - 1 - t))
-        int a = 0, b = m - 2 - tid - r;
-        if (tid > 0) {
-          a = tid - 1 - r;
-          a += 1 + (a < 0 ? m - 1 : 0);
-        }
-        b += 1 + (b < 0 ? m - 1 : 0);
-        const int p = min(a, b), q = max(a, b);
+        int p, q;
+        round_pair(tid, r, m, p, q);
         const R app = A[tri(p, p)], aqq = A[tri(q, q)], apq = A[tri(q, p)];
         float tan;
         if constexpr (k32) {
@@ -198,12 +216,7 @@ __device__ void jacobi_sweeps(R* A, R* V, int ld, int n, int m, Planes<R>& sh, R
             add_low(A[tri(p, p)], sh.low[p], -x);
             add_low(A[tri(q, q)], sh.low[q], x);
           } else {
-            // as updates: their rounding scales with the angle, not with the diagonal
-            const R b = A[tri(q, p)], d = A[tri(p, p)] - A[tri(q, q)];
-            const R cs = fma(-h, s, R(1)) * s, ss = s * s, x = fma(ss, d, R(2) * cs * b);
-            A[tri(q, p)] = fma(cs, d, fma(R(-2) * ss, b, b));
-            A[tri(p, p)] -= x;
-            A[tri(q, q)] += x;
+            turn_plane(h, s, A[tri(p, p)], A[tri(q, p)], A[tri(q, q)]);
           }
         }
       }
@@ -411,11 +424,14 @@ __device__ __forceinline__ int ascending_rank(const double* A, int n, int j) {
 
 // Eigenvalues ascending at base + offE, eigenvectors in descending order at base + offU,
 // each with the sign that makes its largest-magnitude entry (the first one on ties)
-// positive -- the layout launch_reverse_columns produces. A is diagonal, times `scale`.
+// positive -- the layout launch_reverse_columns produces.
 // Equal eigenvalues (the zeros of a sector with empty blocks) keep the order that a selection
 // sort with exchanges leaves them in, since a cut may fall among them.
-__device__ void write_descending(const EigJob& jb, double* base, const double* A, const double* V, double scale,
-                                 int* order) {
+// diag(j): the eigenvalue times `scale`; vec(i, j): element i of its vector. The CTA writes
+// every `parts`-th column from `part` on.
+template <class Diag, class Vec>
+__device__ void write_descending(const EigJob& jb, double* base, Diag diag, Vec vec, double scale, int* order,
+                                 int part = 0, int parts = 1) {
   const int n = jb.n, tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
   if (tid < 32) {
     for (int i = lane; i < n; i += 32) order[i] = i;
@@ -424,7 +440,7 @@ __device__ void write_descending(const EigJob& jb, double* base, const double* A
       double best = 0.0;
       int at = n;
       for (int j = i + lane; j < n; j += 32) {
-        const double v = A[tri(order[j], order[j])];
+        const double v = diag(order[j]);
         if (at == n || v < best) {
           best = v;
           at = j;
@@ -449,14 +465,15 @@ __device__ void write_descending(const EigJob& jb, double* base, const double* A
     }
   }
   __syncthreads();
-  for (int j = tid; j < n; j += blockDim.x) base[jb.offE + j] = A[tri(order[j], order[j])] / scale;
-  for (int o = tid >> 5; o < n; o += nw) {
-    const double* col = V + v_ld(n) * order[n - 1 - o];
+  if (part == 0)
+    for (int j = tid; j < n; j += blockDim.x) base[jb.offE + j] = diag(order[j]) / scale;
+  for (int o = parts * (tid >> 5) + part; o < n; o += parts * nw) {
+    const int col = order[n - 1 - o];
     double best = -1.0, v = 0.0;
     int at = n;
     for (int i = lane; i < n; i += 32)
-      if (fabs(col[i]) > best) {
-        v = col[i];
+      if (const double x = vec(i, col); fabs(x) > best) {
+        v = x;
         best = fabs(v);
         at = i;
       }
@@ -470,7 +487,7 @@ __device__ void write_descending(const EigJob& jb, double* base, const double* A
       }
     }
     const double sgn = v < 0.0 ? -1.0 : 1.0;
-    for (int i = lane; i < n; i += 32) base[jb.offU + i + static_cast<int64_t>(n) * o] = sgn * col[i];
+    for (int i = lane; i < n; i += 32) base[jb.offU + i + static_cast<int64_t>(n) * o] = sgn * vec(i, col);
   }
 }
 
@@ -540,7 +557,8 @@ __device__ __forceinline__ void gram_eigen(const EigJob& jb, double* base, doubl
   }
   __syncthreads();
   if (n > 1) jacobi_sweeps<double>(A, V, ld, n, m, sh, 1e-30, 30);
-  write_descending(jb, base, A, V, sc, order);
+  write_descending(
+      jb, base, [=](int j) { return A[tri(j, j)]; }, [=](int i, int j) { return V[i + ld * j]; }, sc, order);
 }
 
 // order <= kBatchedEigMax
@@ -554,7 +572,8 @@ __global__ void __launch_bounds__(kEigSmallThreads, 1) batched_eig_kernel(const 
   gram_eigen(jobs[blockIdx.x], base, A, V, sh, order);
 }
 
-// order kBatchedEigMax + 1 .. kBatchedEigLargeMax: A and V in dynamic shared memory
+// order kBatchedEigMax + 1 .. kBatchedEigLargeMax, many matrices: A and V in dynamic shared
+// memory
 constexpr int kEigLargeThreads = 512;
 __host__ __device__ constexpr size_t eig_large_bytes(int n) {
   return sizeof(double) * (static_cast<size_t>(tri_size(even_up(n))) + static_cast<size_t>(even_up(n)) * v_ld(n));
@@ -566,6 +585,200 @@ __global__ void __launch_bounds__(kEigLargeThreads) batched_eig_large_kernel(con
   __shared__ int order[kBatchedEigLargeMax];
   const EigJob jb = jobs[blockIdx.x];
   gram_eigen(jb, base, dyn, dyn + tri_size(even_up(jb.n)), sh, order);
+}
+
+// The same orders, few matrices: a cluster of kCl CTAs for each, the
+// same sweeps. In one CTA a round at order 128 is 49000 FP64 operations at 1.6 a clock
+// (15 us) while nearly all SMs have nothing to do, as a state has few sectors of this size.
+// Element e of the packed A is in CTA e mod kCl (in two copies: a round reads one and writes
+// all of the other, so that it needs one cluster barrier), V's rows are dealt out in
+// ranges, and every CTA finds all rotations of a round itself. V is turned between the
+// arrival at the barrier and the wait. Now a round's chain bounds it (rotations from remote
+// elements, blocks, barrier: 1 to 5 us).
+constexpr int kCl = 8, kClThreads = 256;
+// While two of its CTAs fit an SM the cluster is the faster one; ms for one CTA -> cluster, Gaussian
+// spectrum: 6 matrices order 33 0.61 -> 0.52, 48 1.22 -> 0.77, 64 2.85 -> 1.21, 96 9.0 -> 2.7, 128
+// 20.3 -> 5.1; 38 matrices 0.55 -> 0.58, 1.23 -> 1.10, 2.86 -> 1.79, 9.0 -> 5.3, 20.9 -> 11.7; 60
+// matrices 0.55 -> 1.16, 1.24 -> 1.97, 2.85 -> 3.24, 8.6 -> 9.4, 20.6 -> 19.5. (512 threads: 4.8 ms for
+// one of order 128 instead of 5.2, but half as many at a time; four CTAs: 7.9 ms.)
+constexpr int kClMaxJobs = 38;
+constexpr int kClA = (tri_size(kBatchedEigLargeMax) + kCl - 1) / kCl;
+constexpr int kClRows = (kBatchedEigLargeMax + kCl - 1) / kCl, kClLd = kClRows + 1;
+
+__device__ __forceinline__ uint32_t cl_addr(uint32_t a, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ double cl_load(uint32_t a, int rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cl_addr(a, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cl_store(uint32_t a, int rank, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cl_addr(a, rank)), "d"(v) : "memory");
+}
+// (the barrier's instructions are for whole warps)
+__device__ __forceinline__ void cl_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cl_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cl_sync() {
+  cl_arrive();
+  cl_wait();
+}
+
+__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kClThreads, 1)
+    batched_eig_cluster_kernel(const EigJob* __restrict__ jobs, double* __restrict__ base) {
+  __shared__ double A[2][kClA], V[kBatchedEigLargeMax * kClLd];
+  __shared__ double H[2][kBatchedEigLargeMax / 2], S[2][kBatchedEigLargeMax / 2];  // by parity of the round
+  __shared__ int Pl[2][kBatchedEigLargeMax / 2], Ql[2][kBatchedEigLargeMax / 2];
+  __shared__ double red[2][32], part[2], lam[kBatchedEigLargeMax];
+  __shared__ int order[kBatchedEigLargeMax];
+  const EigJob jb = jobs[blockIdx.x / kCl];
+  const int rank = blockIdx.x % kCl;  // in the cluster too: clusters are runs of kCl CTAs
+  const int n = jb.n, m = even_up(n), npair = m / 2, nel = tri_size(m), nblk = npair * (npair - 1) / 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (n + kCl - 1) / kCl, row0 = rank * per, nrow = max(0, min(per, n - row0));
+  const uint32_t a0 = static_cast<uint32_t>(__cvta_generic_to_shared(&A[0][0]));
+  auto at = [&](int b, int e) { return a0 + static_cast<uint32_t>(8 * (b * kClA + e / kCl)); };
+  auto get = [&](int b, int e) { return cl_load(at(b, e), e % kCl); };
+  auto put = [&](int b, int e, double v) { cl_store(at(b, e), e % kCl, v); };
+
+  const double* G = base + jb.offG;
+  double big = 0.0;
+  for (int e = tid; e < n * n; e += kClThreads) big = fmax(big, fabs(G[e]));
+  const double sc = unit_scale(big, red[0]), hs = 0.5 * sc;
+  for (int e = tid; e < m * m; e += kClThreads) {
+    const int i = e % m, j = e / m, x = tri(i, j);
+    if (j <= i && x % kCl == rank) A[0][x / kCl] = i < n ? hs * G[i + n * j] + hs * G[j + n * i] : 0.0;
+  }
+  for (int e = tid; e < m * kClLd; e += kClThreads) V[e] = row0 + e % kClLd == e / kClLd ? 1.0 : 0.0;
+  cl_sync();
+
+  // this thread's 2 x 2 block (planes bP < bQ of a cycle, each pair once) and the first of
+  // its elements of V with the steps to the next
+  static_assert(kBatchedEigLargeMax / 2 * (kBatchedEigLargeMax / 2 - 1) / 2 <= kCl * kClThreads, "a block a thread");
+  const int blk = rank + kCl * tid, bP = blk % npair, bQ0 = bP + 1 + blk / npair;
+  const int bQ = bQ0 < npair ? bQ0 : bQ0 - npair;
+  const bool block = blk < nblk;
+  const int rows = max(nrow, 1), i0 = tid % rows, W0 = nrow > 0 ? tid / rows : npair;
+  const int dI = kClThreads % rows, dW = kClThreads / rows;
+
+  int cur = 0, par = 0;
+  double goal = 0.0;
+  for (int sweep = 0; sweep < 30 && n > 1; sweep++) {
+    // off(A)^2 and |A|^2: every CTA adds the same eight parts in the same order, so that all
+    // of the cluster take the same way
+    double off = 0.0, tot = 0.0;
+    for (int s = tid; s * kCl + rank < nel; s += kClThreads) {
+      const int e = s * kCl + rank;
+      int i = static_cast<int>((sqrtf(8.0f * static_cast<float>(e) + 1.0f) - 1.0f) * 0.5f);
+      while (tri_size(i + 1) <= e) i++;
+      while (tri_size(i) > e) i--;
+      const double v = A[cur][s];
+      if (e - tri_size(i) == i) tot += v * v;
+      else off += v * v;
+    }
+    off *= 2.0;
+    tot += off;
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_down_sync(0xffffffffu, off, o);
+      tot += __shfl_down_sync(0xffffffffu, tot, o);
+    }
+    if (lane == 0) {
+      red[0][warp] = off;
+      red[1][warp] = tot;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      double v = 0.0;
+      for (int w = 0; w < kClThreads / 32; w++) v += red[tid][w];
+      part[tid] = v;
+    }
+    cl_sync();
+    off = tot = 0.0;
+    const uint32_t pa = static_cast<uint32_t>(__cvta_generic_to_shared(part));
+    for (int c = 0; c < kCl; c++) {
+      off += cl_load(pa, c);
+      tot += cl_load(pa + 8, c);
+    }
+    if (sweep == 0) goal = 1e-30 * tot;
+    if (!(off > goal)) break;
+    for (int r = 0; r < m - 1; r++) {
+      const int nxt = cur ^ 1;
+      if (tid < npair) {
+        int p, q;
+        round_pair(tid, r, m, p, q);
+        const double app = get(cur, tri(p, p)), aqq = get(cur, tri(q, q)), apq = get(cur, tri(q, p));
+        float tan;
+        const float hf = half_tangent(d2f(aqq - app), d2f(apq), tan);
+        const double h = f2d(hf);
+        H[par][tid] = h;
+        S[par][tid] = sine(h, hf);
+        Pl[par][tid] = p;
+        Ql[par][tid] = q;
+      }
+      __syncthreads();
+      if (const int P = rank + kCl * (kClThreads - 1 - tid); P < npair) {
+        const int p = Pl[par][P], q = Ql[par][P], pp = tri(p, p), qp = tri(q, p), qq = tri(q, q);
+        double a = get(cur, pp), b = get(cur, qp), d = get(cur, qq);
+        turn_plane(H[par][P], S[par][P], a, b, d);
+        put(nxt, pp, a);
+        put(nxt, qp, b);
+        put(nxt, qq, d);
+      }
+      if (block) {
+        const int P = bP, Q = bQ;
+        const double hp = H[par][P], sp = S[par][P], hq = H[par][Q], sq = S[par][Q];
+        const int p = Pl[par][P], q = Ql[par][P], u = Pl[par][Q], v = Ql[par][Q];
+        const int pu = tri(p, u), pv = tri(p, v), qu = tri(q, u), qv = tri(q, v);
+        double a = get(cur, pu), b = get(cur, pv), c = get(cur, qu), d = get(cur, qv);
+        rotate(hp, sp, a, c);
+        rotate(hp, sp, b, d);
+        rotate(hq, sq, a, b);
+        rotate(hq, sq, c, d);
+        put(nxt, pu, a);
+        put(nxt, pv, b);
+        put(nxt, qu, c);
+        put(nxt, qv, d);
+      }
+      cl_arrive();
+      for (int i = i0, P = W0; P < npair;) {
+        const double h = H[par][P], s = S[par][P];
+        if (s != 0.0) {
+          double* vp = V + kClLd * Pl[par][P] + i;
+          double* vq = V + kClLd * Ql[par][P] + i;
+          double x = *vp, y = *vq;
+          rotate(h, s, x, y);
+          *vp = x;
+          *vq = y;
+        }
+        i += dI;
+        P += dW;
+        if (i >= nrow) {
+          i -= nrow;
+          P++;
+        }
+      }
+      cl_wait();
+      // the next round's planes go to the other copy: V may still be turned by these
+      cur = nxt;
+      par ^= 1;
+    }
+  }
+  for (int j = tid; j < n; j += kClThreads) lam[j] = get(cur, tri(j, j));
+  cl_sync();  // all rows of V are final
+  const uint32_t v0 = static_cast<uint32_t>(__cvta_generic_to_shared(V));
+  write_descending(
+      jb, base, [&](int j) { return lam[j]; },
+      [&](int i, int j) { return cl_load(v0 + static_cast<uint32_t>(8 * (kClLd * j + i % per)), i / per); }, sc, order,
+      rank, kCl);
+  cl_sync();  // no CTA ends while another reads its rows
 }
 
 // Loewdin orthonormaliser of k <= 4 vectors: L = S^-1/2 from the k x k overlap S
@@ -635,11 +848,14 @@ cudaError_t launch_batched_eig(const EigJob* jobs, int njobs, double* base, cuda
 cudaError_t launch_batched_eig_large(const EigJob* jobs, int njobs, int nmax, double* base, cudaStream_t stream) {
   if (njobs <= 0) return cudaSuccess;
   if (nmax > kBatchedEigLargeMax) return cudaErrorInvalidValue;
-  const size_t bytes = eig_large_bytes(nmax);
+  if (njobs <= kClMaxJobs) {
+    batched_eig_cluster_kernel<<<kCl * njobs, kClThreads, 0, stream>>>(jobs, base);
+    return cudaGetLastError();
+  }
   const cudaError_t e = cudaFuncSetAttribute(batched_eig_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(eig_large_bytes(kBatchedEigLargeMax)));
   if (e != cudaSuccess) return e;
-  batched_eig_large_kernel<<<njobs, kEigLargeThreads, bytes, stream>>>(jobs, base);
+  batched_eig_large_kernel<<<njobs, kEigLargeThreads, eig_large_bytes(nmax), stream>>>(jobs, base);
   return cudaGetLastError();
 }
 
