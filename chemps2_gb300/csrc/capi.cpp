@@ -782,6 +782,96 @@ int c2g_rayleigh_ritz_eig(int n, const double* mat, int warm, double* evals, dou
   });
 }
 
+int c2g_two_pass_products(int digits, int m, int n, int k, int count, int trans, int splits, const double* l,
+                          const double* r, const double* alpha, double* products, double* sum) {
+  return guarded([&] {
+    if (m < 1 || n < 1 || k < 1 || m > 4096 || n > 4096 || k > 4096 || count < 1 || count > 4096 || splits < 1 ||
+        splits > count || trans < 0 || trans > 3)
+      throw std::invalid_argument("c2g_two_pass_products: argument out of range");
+    NEED(l);
+    NEED(r);
+    NEED(alpha);
+    NEED(products);
+    NEED(sum);
+    const int64_t ml = static_cast<int64_t>(m) * k, mr = static_cast<int64_t>(k) * n, mp = static_cast<int64_t>(m) * n;
+    std::vector<c2g::InterJob> jobs(count);
+    std::vector<c2g::SumItem> items(count);
+    std::vector<c2g::GemmTile> jtiles, stiles;
+    for (int i = 0; i < count; i++) {
+      c2g::InterJob& J = jobs[i];
+      J.l = {c2g::make_ref(c2g::kSlotX, ml * i), (trans & 1) ? k : m, trans & 1};
+      J.r = {c2g::make_ref(c2g::kSlotCombo, mr * i), (trans & 2) ? n : k, trans >> 1};
+      J.m = m;
+      J.n = n;
+      J.k = k;
+      J.off = mp * i;
+      items[i].l = J.l;
+      items[i].r = J.r;
+      items[i].alpha = alpha[i];
+      items[i].k = k;
+    }
+    const c2g::SumGroup group{c2g::make_ref(c2g::kSlotY, 0), m, n, m, 0, 0, count};
+    for (int i = 0; i < (m + 63) / 64; i++)
+      for (int j = 0; j < (n + 63) / 64; j++) {
+        c2g::GemmTile t{};
+        t.pos = i << 16 | j;
+        t.shape = ((std::min(64, m - 64 * i) + 15) / 16 - 1) | ((std::min(64, n - 64 * j) + 15) / 16 - 1) << 2;
+        t.nsplit = 1;
+        for (t.idx = 0; t.idx < count; t.idx++) jtiles.push_back(t);
+        t.idx = 0;
+        t.nsplit = splits;
+        t.counter = static_cast<int>(stiles.size()) / splits;
+        t.part = static_cast<int64_t>(4096) * stiles.size();
+        for (t.split = 0; t.split < splits; t.split++) {
+          t.item0 = static_cast<int>(static_cast<int64_t>(count) * t.split / splits);
+          t.item1 = static_cast<int>(static_cast<int64_t>(count) * (t.split + 1) / splits);
+          stiles.push_back(t);
+        }
+      }
+    std::vector<void*> held;
+    struct Free {
+      std::vector<void*>& p;
+      ~Free() {
+        for (void* q : p) cudaFree(q);
+      }
+    } guard_free{held};
+    auto put = [&](const void* src, size_t bytes) {
+      void* p = nullptr;
+      C2G_CUDA(cudaMalloc(&p, bytes));
+      held.push_back(p);
+      if (src) C2G_CUDA(cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice));
+      else C2G_CUDA(cudaMemset(p, 0, bytes));
+      return p;
+    };
+    c2g::SlotPtrs sp{};
+    sp.x = static_cast<double*>(put(l, 8 * ml * count));
+    sp.combo = static_cast<double*>(put(r, 8 * mr * count));
+    sp.y = static_cast<double*>(put(nullptr, 8 * mp));
+    sp.inter = static_cast<double*>(put(nullptr, 8 * mp * count));
+    auto* dj = static_cast<c2g::InterJob*>(put(jobs.data(), sizeof(jobs[0]) * jobs.size()));
+    auto* di = static_cast<c2g::SumItem*>(put(items.data(), sizeof(items[0]) * items.size()));
+    auto* dg = static_cast<c2g::SumGroup*>(put(&group, sizeof(group)));
+    auto* djt = static_cast<c2g::GemmTile*>(put(jtiles.data(), sizeof(jtiles[0]) * jtiles.size()));
+    auto* dst = static_cast<c2g::GemmTile*>(put(stiles.data(), sizeof(stiles[0]) * stiles.size()));
+    auto* part = static_cast<double*>(put(nullptr, 8 * 4096 * stiles.size()));
+    auto* words = static_cast<unsigned*>(put(nullptr, 4 * (5 + stiles.size())));  // scheduler, error, counters
+    int* err = reinterpret_cast<int*>(words + 4);
+    const int nj = static_cast<int>(jtiles.size()), ns = static_cast<int>(stiles.size());
+    if (digits) {
+      C2G_CUDA(c2g::launch_inter_digits(dj, djt, nj, sp, words, err, nullptr));
+      C2G_CUDA(c2g::launch_sum_digits(dg, di, dst, ns, part, words + 5, sp, words + 2, err, nullptr));
+    } else {
+      C2G_CUDA(c2g::launch_inter_gemm(dj, djt, nj, sp, nullptr, c2g::Precision::kFP64));
+      C2G_CUDA(c2g::launch_sum_gemm(dg, di, dst, ns, part, words + 5, sp, nullptr, c2g::Precision::kFP64));
+    }
+    C2G_CUDA(cudaMemcpy(products, sp.inter, 8 * mp * count, cudaMemcpyDeviceToHost));
+    C2G_CUDA(cudaMemcpy(sum, sp.y, 8 * mp, cudaMemcpyDeviceToHost));
+    int e = 0;
+    C2G_CUDA(cudaMemcpy(&e, err, sizeof(e), cudaMemcpyDeviceToHost));
+    if (e) throw std::runtime_error("c2g_two_pass_products: a kernel gave up a wait");
+  });
+}
+
 int c2g_device_memory_info(int device, int64_t* free_bytes, int64_t* pool_used_bytes) {
   return guarded([&] {
     NEED(free_bytes);

@@ -8,38 +8,44 @@
 //
 // A step is one product L (m x K) R (K x n) of at most 64 x 32 outputs and K <= 32. Each row
 // of L and column of R is scaled by the power of two above its largest magnitude, 2^e, and
-// every element becomes the integer X = v 2^(55 - e) to the nearest, |X| <= 2^55: seven
-// digits to the base 256, the first in [-128, 128], the others in [-128, 127], so exact in
-// FP16. (One scale for a whole block would do for norms, but not for the small rows and columns
-// of a vector graded by its singular values: their errors came out up to three times the FP64
-// pipe's.) The tensor core sums d_i d_j over K and over the pairs of one diagonal c = i + j <= 7
-// in FP32: at most 7 x 64 products of at most 2^14, below 2^24, so every sum is exact. Dropped
-// are the diagonals c >= 8, about 2^-64 of the largest product. The eight sums are put
-// together in 64-bit integers and rounded to a double by integer instructions; one FP64
-// instruction adds that to the item sum, where the FP64 pipe rounds at each of the K terms.
-// Products longer than 32 take several steps; a second one adds to the first one's sums in
-// tensor memory where its elements fit the same scales, and else to its rounded ones.
-// Measured against extended precision, random operands of one size or spread over 2^20: pass
-// 1 0.4 to 1.0e-16 of the norm (FP64 pipe 1.0 to 2.6e-16), pass 2 with 200 items 2.0 to 5.9e-16
-// (one rounding of each FP64-summed item: 2.9 to 7.8e-16).
+// every element becomes the integer X = v 2^(62 - e) to the nearest, |X| <= 2^62: eight digits
+// to the base 256 in [-128, 127], exact in FP16. The tensor core sums d_i d_j over K and over
+// the pairs of one diagonal c = i + j <= 7 in FP32: at most 8 x 64 products of at most 2^14, so
+// below 2^24 and exact. Dropped are the diagonals c >= 8. The eight sums are put together in
+// 96 bits and rounded to a double by integer instructions; one FP64 instruction adds that to
+// the item sum, where the FP64 pipe rounds at each of the K terms. Products longer than 32 take
+// several steps; a second one adds to the first one's sums in tensor memory where its elements
+// fit the same scales, and else to its rounded ones.
+//
+// What is dropped is small beside M, the product of the row's and the column's scales (at most
+// K 2^-59 M, 2^-62 M as a rule), and so beside an output of which a product is near M, but not
+// beside one where L is large along K where R is small, and the other way round. So each
+// element has a weight, the binary orders d that it is below its row's or column's largest,
+// and an output is taken from the digits only where some k has d <= 1, 3 or 5 in L and d <= 5, 3
+// or 1 in R (a product of 2^-8 M or more), or no product at all. Any other one is formed by the K
+// FP64 multiply-adds of the FP64 pipe. rms errors in units of 2^-53 sum |l| |r|, digits / FP64
+// pipe: operands of one size 0.12 to 0.18 / 0.46 to 0.49, spread over 2^40 0.8 to 1.1 / 1.0 to 2.3, L
+// falling and R rising along K by 2, 6 and 20 decades 0.12 to 0.30, 0.18 to 0.47 and 0.29 to 0.48 / 0.44
+// to 0.49. Outputs formed by multiply-adds: none of random operands; in swept states 0.2 to 6 %
+// of pass 1's and 0.01 to 0.5 % of pass 2's (ab initio to Hubbard L = 16).
 //
 // L's digits are rows of shared memory digit by digit and so are R's columns, so that digit i
-// of L meets digits 0 .. 7 - i of R in one MMA whose accumulator starts at column group i
-// (an eighth digit of R, of zeros, sets the last diagonal): 7 MMAs of M = 128 for each 16 of
-// K. Persistent 256-thread CTAs, two per SM (256 columns of tensor memory each, and 87 KB of
-// shared memory in pass 1, 104 in pass 2, so that one cuts digits and rounds sums while the
+// of L meets digits 0 .. 7 - i of R in one MMA whose accumulator starts at column group i: 8
+// MMAs of M = 128 for each 16 of K. Persistent 256-thread CTAs, two per SM (256 columns of
+// tensor memory and 110 KB of shared memory each, so that one cuts digits and rounds sums while the
 // other's MMAs run) take the 64 x 32 halves of the tile lists' tiles from an atomic counter.
 // While the MMAs of a step run, all threads round the previous step's sums (copied from
 // tensor memory to shared memory by the warps of the quadrants that hold them) and the next
 // step's operands are on their way from memory. An operand that the step before had too is
 // not cut again.
 //
-// What bounds it: a step's fixed chain, load - exponents - digits - MMA - collect, of 2.1 to
-// 4 us an SM whatever its size, with the tensor pipe busy a fifth to a quarter of the time and
+// What bounds it: a step's fixed chain, load - exponents - digits - MMA - collect, of 2.2 to
+// 4.6 us an SM whatever its size, with the tensor pipe busy a fifth to a quarter of the time and
 // the issue slots 35 to 40 %. us a product and SM, FP64 pipe -> digits, pass 1 / pass 2:
-// 17 x 17 x 17 3.1 -> 2.4 / 4.2 -> 3.3, 32 x 32 x 32 8.3 -> 3.0 / 10.0 -> 4.3, 47 x 47 x 47 27 -> 9.0 /
-// 31 -> 10.6, 64 x 64 x 64 65 -> 12.2 / 73 -> 13.7. Below about 17 x 17 x 12 the FP64 pipe is the
-// faster one (digits_pay in runtime.cpp).
+// 17 x 17 x 17 3.1 -> 2.7 / 4.2 -> 3.6, 32 x 32 x 32 8.3 -> 3.3 / 10.0 -> 4.6, 47 x 47 x 47 27 -> 11.0 /
+// 31 -> 11.7, 64 x 64 x 64 65 -> 14.8 / 73 -> 15.5. With seven digits and no weights the last three were
+// 3.0 / 4.4, 9.1 / 10.6 and 12.2 / 13.7, but outputs without a product near M lost up to all of their
+// digits. Below about 17 x 17 x 12 the FP64 pipe is the faster one (digits_pay in runtime.cpp).
 //
 // Every mbarrier wait is bounded: after kTcSpinLimit polls the kernel records an error in
 // the runtime's mapped error word, frees its tensor memory and returns without writing its
@@ -62,7 +68,7 @@ constexpr int kDgThreads = 256;
 constexpr int kDgIssuer = 5;  // the warp that issues the MMAs: of the last to cut digits, and
                               // without tile rows of tensor memory in a tile of 32 rows
 constexpr int kDgCtasPerSm = 2;
-constexpr int kDgDigits = 7, kDgDiagonals = 8;
+constexpr int kDgDigits = 8, kDgDiagonals = kDgDigits;
 constexpr int kDgRows = 64, kDgCols = 32, kDgK = 32;  // of a step
 constexpr uint32_t kDgTmemCols = kDgDiagonals * kDgCols;
 constexpr int kDgBatch = 32;                          // records held in shared memory
@@ -71,7 +77,7 @@ constexpr int kDgBatch = 32;                          // records held in shared 
 // between the two 8-wide halves of K
 constexpr int kDgRowBytes = 32;
 constexpr int kDgLBytes = kDgDigits * kDgRows * kDgRowBytes;  // one half (16) of a step's K
-constexpr int kDgRBytes = (kDgDigits + 1) * kDgCols * kDgRowBytes;  // with a digit of zeros
+constexpr int kDgRBytes = kDgDigits * kDgCols * kDgRowBytes;
 // leading dimension of a row of sums: 16-byte accesses of eight rows meet every bank once
 constexpr int kDgSumLd = kDgCols + 4;
 
@@ -89,6 +95,14 @@ struct DgRecord {  // 64 bytes
 };
 static_assert(sizeof(DgRecord) == 64, "DgRecord");
 
+// A step whose sums are not rounded yet: its product's record, its range of K (up to two
+// steps') and whether that begins and ends the product.
+struct DgStep {
+  DgRecord x;
+  int32_t k0, k1;
+  bool first, last;
+};
+
 struct __align__(1024) DgSmem {
   unsigned char l[2 * kDgLBytes];
   unsigned char r[2 * kDgRBytes];
@@ -98,9 +112,13 @@ struct __align__(1024) DgSmem {
   // largest exponent fields of the rows of L, then of the columns of R: of the step in
   // flight, the one being staged and (zero) the next
   alignas(16) unsigned int expo[3][kDgRows + kDgCols];
+  // weight words (dg_weight) of the rows of L, then of the columns of R, by groups of 8 of K
+  uint4 weight[kDgRows + kDgCols];
+  DgStep step[2];  // of the step in flight and the next
   uint32_t tmem_base;
   int slot, is_last;
-  // pass 2: a product's sums over its first steps, each thread's own outputs
+  // each thread's own outputs: in pass 2 a product's sums over its first steps, in pass 1 what
+  // is formed by multiply-adds
   double part[8][kDgThreads];
 };
 
@@ -134,26 +152,40 @@ __device__ __forceinline__ unsigned int dg_exponent(const DgUnit& u) {
   return e >> 20;
 }
 
-// X + sum_i 128 256^i of an element: its digits less their sign, as bytes (the first digit as
-// nine bits); emax: the row's largest exponent field
+// X + sum_i 128 256^i of an element: its eight digits plus 128, as bytes; emax: the row's
+// largest exponent field
 __device__ __forceinline__ unsigned long long dg_fixed(double v, unsigned int emax) {
   const unsigned int hi = __double2hiint(v), lo = __double2loint(v);
   const unsigned int e = (hi >> 20) & 0x7ffu;
   const unsigned long long m =
-      (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 3;  // below 2^56
+      (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;  // below 2^63
   const unsigned int sh = e == 0u ? 63u : min(emax - e, 63u);
-  const unsigned long long x = ((m >> sh) + 1ull) >> 1;  // to the nearest, below 2^55
+  const unsigned long long x = ((m >> sh) + 1ull) >> 1;  // to the nearest, below 2^62
   const unsigned long long s = static_cast<long long>(static_cast<int>(hi)) >> 63;
-  return (x ^ s) - s + 0x0080808080808080ull;
+  return (x ^ s) - s + 0x8080808080808080ull;
+}
+
+// How far a unit's elements are below the row's largest, in binary orders d: bit k of byte
+// 0 is set where the element is not zero, of byte 1 where d <= 5, of byte 2 where d <= 3 and
+// of byte 3 where d <= 1.
+__device__ __forceinline__ uint32_t dg_weight(const DgUnit& u, unsigned int emax) {
+  uint32_t w = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const unsigned int hi = __double2hiint(u.v[k]), lo = __double2loint(u.v[k]);
+    const unsigned int d = min(emax - ((hi >> 20) & 0x7ffu), 6u);
+    const uint32_t t = (0x01010101u << k) >> ((4u * d) & 24u);
+    if (((hi & 0x7fffffffu) | lo) != 0u) w |= t;
+  }
+  return w;
 }
 
 // digit i of two such integers as FP16, low first: 1024 + byte in FP16, less 1152
 template <int i>
 __device__ __forceinline__ uint32_t dg_pair(unsigned long long a, unsigned long long b) {
-  constexpr int byte = (6 - i) & 3;
-  const uint32_t x = static_cast<uint32_t>(i < 3 ? a >> 32 : a), y = static_cast<uint32_t>(i < 3 ? b >> 32 : b);
-  const uint32_t t = i == 0 ? __byte_perm(x, y, 0x7632) | 0x64006400u
-                            : (__byte_perm(x, y, byte | (4 + byte) << 8) & 0x00ff00ffu) | 0x64006400u;
+  constexpr int byte = (7 - i) & 3;
+  const uint32_t x = static_cast<uint32_t>(i < 4 ? a >> 32 : a), y = static_cast<uint32_t>(i < 4 ? b >> 32 : b);
+  const uint32_t t = (__byte_perm(x, y, byte | (4 + byte) << 8) & 0x00ff00ffu) | 0x64006400u;
   const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&t), __floats2half2_rn(1152.0f, 1152.0f));
   return *reinterpret_cast<const uint32_t*>(&h);
 }
@@ -177,23 +209,47 @@ __device__ __forceinline__ void dg_store(const DgUnit& u, unsigned int emax, uns
   C2G_DIGIT(4)
   C2G_DIGIT(5)
   C2G_DIGIT(6)
+  C2G_DIGIT(7)
 #undef C2G_DIGIT
 }
 
-// n 2^k as a double to the nearest, by the bits (a conversion or an FP64 instruction costs a
-// warp 65 clocks): zero where the result is below the normal range, infinite above it.
-__device__ __forceinline__ double rounded(long long n, int k) {
-  const unsigned long long s = static_cast<unsigned long long>(n >> 63);
-  unsigned long long u = (static_cast<unsigned long long>(n) ^ s) - s;
-  const int z = __clzll(static_cast<long long>(u));
-  u <<= z & 63;
-  const unsigned int hs = static_cast<unsigned int>(s) & 0x80000000u;
-  const int f = 1086 - z + k;  // the exponent field
-  if (u == 0ull || f <= 0) return __hiloint2double(hs, 0);
-  if (f >= 0x7fe) return __hiloint2double(hs | 0x7ff00000u, 0);
-  const unsigned long long m = (u + 0x400ull < u) ? 1ull << 53 : (u + 0x400ull) >> 11;  // 2^52 .. 2^53
+// (hi 2^32 + lo) 2^k as a double to the nearest, by the bits (a conversion or an FP64
+// instruction costs a warp 65 clocks); |hi| < 2^62, |lo| < 2^62. A negative one is off by a unit
+// of lo before it is rounded. Zero where the result is below the normal range, infinite above it.
+__device__ __forceinline__ double rounded(long long hi, long long lo, int k) {
+  hi += lo >> 32;
+  const unsigned int s = static_cast<unsigned int>(hi >> 63);
+  const unsigned int h2 = static_cast<unsigned int>(hi >> 32) ^ s, h1 = static_cast<unsigned int>(hi) ^ s,
+                     h0 = static_cast<unsigned int>(lo) ^ s;
+  // the 96 bits h, normalised
+  const bool a = h2 == 0u, b = a && h1 == 0u;
+  const unsigned int w2 = b ? h0 : a ? h1 : h2, w1 = b ? 0u : a ? h0 : h1, w0 = a ? 0u : h0;
+  const int z = __clz(static_cast<int>(w2));
+  const int f = 1086 + 32 + k - z - (b ? 64 : a ? 32 : 0);  // the exponent field
+  const unsigned long long u =
+      static_cast<unsigned long long>(__funnelshift_l(w1, w2, z)) << 32 | __funnelshift_l(w0, w1, z);
+  const unsigned long long m = (u >> 11) + ((u >> 10) & 1u);  // 2^52 .. 2^53
   const unsigned long long v = (static_cast<unsigned long long>(f - 1) << 52) + m;
-  return __hiloint2double(hs | static_cast<unsigned int>(v >> 32), static_cast<unsigned int>(v));
+  const unsigned int top = static_cast<unsigned int>(v >> 32) | (s & 0x80000000u);
+  if (w2 == 0u || f <= 0) return 0.0;
+  if (f >= 0x7fe) return __hiloint2double((s & 0x80000000u) | 0x7ff00000u, 0);
+  return __hiloint2double(top, static_cast<unsigned int>(v));
+}
+
+// Output (i, j) of a step by FP64 multiply-adds.
+__device__ __forceinline__ double dg_direct(const DgStep& S, int i, int j) {
+  const DgRecord& X = S.x;
+  const int64_t ls = X.ltrans ? 1 : X.lld, rs = X.rtrans ? 1 : X.rld;
+  const double* l = X.l + (X.ltrans ? static_cast<int64_t>(X.lld) * i : i) + ls * S.k0;
+  const double* r = X.r + (X.rtrans ? static_cast<int64_t>(X.rld) * j : j) + rs * S.k0;
+  double v = 0.0;
+#pragma unroll 4
+  for (int k = S.k1 - S.k0; k > 0; k--) {
+    v = fma(*l, *r, v);
+    l += ls;
+    r += rs;
+  }
+  return v;
 }
 
 __device__ __forceinline__ bool elect_one() {
@@ -233,8 +289,8 @@ struct DgEngine {
   uint32_t phase = 0u;
   bool flying = false, ok = true;
   int held = 0, cur = 1;  // exponent tables of the step in flight and of the one being staged
-  double alpha = 0.0;     // pass 2: of the step in flight
-  // the sums so far: row, columns col .. col + outputs - 1
+  int at = 0;             // record of the step in flight
+  // pass 2: the sums so far, columns col .. of the thread's row
   double acc[8];
 
   __device__ __forceinline__ DgEngine(DgSmem& s) : sm(s), tmem(s.tmem_base) { clear(); }
@@ -248,8 +304,8 @@ struct DgEngine {
     return big ? (threadIdx.x >> 6) * 8 : (threadIdx.x >> 5) * 4;
   }
 
-  // Issues the MMAs of the staged step of 16 `halves` of K (one thread), `onto` the sums there. Digit i of L meets
-  // digits 0 .. 7 - i of R, the eighth of which is zero: it sets the last diagonal's sums.
+  // Issues the MMAs of the staged step of 16 `halves` of K (one thread), `onto` the sums
+  // there. Digit i of L meets digits 0 .. 7 - i of R.
   __device__ __forceinline__ void issue(int halves, bool onto) {
     tc_fence_after();
     const uint64_t a0 = smem_desc(smem_u32(sm.l), 128, 256), b0 = smem_desc(smem_u32(sm.r), 128, 256);
@@ -271,8 +327,9 @@ struct DgEngine {
   }
 
   // Tensor memory -> shared memory: warp w holds rows 32 (w % 4) .. + 31 and columns
-  // 16 (w / 4) .. + 15. Two diagonals make one integer, 256 i_c + i_(c+1), below 2^30.
-  __device__ __forceinline__ void collect(int rows, int cols) {
+  // 16 (w / 4) .. + 15. Two diagonals make one integer, 256 i_c + i_(c+1), below 2^31.
+  __device__ __forceinline__ void collect() {
+    const int rows = sm.step[at].x.rows, cols = sm.step[at].x.cols;
     const int warp = threadIdx.x >> 5, quad = warp & 3, c0 = 16 * (warp >> 2);
     if (quad * 32 < rows && c0 < cols) {
       const uint32_t from = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(c0);
@@ -297,18 +354,22 @@ struct DgEngine {
     tc_fence_before();
   }
 
-  // The collected sums, each rounded once: into acc (kSet), onto it (kAdd), or (kScale) with
-  // those of the product's other steps, times alpha, onto it: an item is rounded into acc
-  // once whatever its inner dimension, as on the FP64 pipe. An infinite or NaN element makes its row's or column's outputs NaN.
-  enum Mode { kSet, kAdd, kScale };
-  template <int kOut, Mode kMode>
-  __device__ __forceinline__ void finish(int rows, int cols, bool first, bool last) {
-    constexpr bool big = kOut == 8;
-    const int r = row_of(big), c0 = col_of(big);
-    if (r >= rows || c0 >= cols) return;
+  // The value of diagonals p in units of 2^e / 2^2044: p0 2^-20 + p1 2^-36 + p2 2^-52 + p3 2^-68
+  __device__ __forceinline__ static double value(int p0, int p1, int p2, int p3, unsigned int el, unsigned int er) {
+    double v = rounded(static_cast<long long>(p0) * 65536 + p1, static_cast<long long>(p2) * 65536 + p3,
+                       static_cast<int>(el + er) - 2044 - 68);
+    if (el == 0x7ffu || er == 0x7ffu) v = __longlong_as_double(0x7ff8000000000000ll);
+    return v;
+  }
+
+  // The collected sums of a whole product, each rounded once: to memory, or times alpha into acc.
+  template <int kOut, bool kEach>
+  __device__ __forceinline__ void finish_whole(const DgStep& S) {
+    const int r = row_of(kOut == 8), c0 = col_of(kOut == 8);
     const int* s = sm.sums + r * kDgSumLd + c0;
     const unsigned int* expo = sm.expo[held];
     const unsigned int el = expo[r];
+    double* to = S.x.s + r + static_cast<int64_t>(S.x.lds) * c0;
 #pragma unroll
     for (int q = 0; q < kOut; q += 4) {
       int p[4][4];
@@ -324,36 +385,97 @@ struct DgEngine {
       const unsigned int er[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
       for (int t = 0; t < 4; t++) {
-        const int k = q + t;
-        // p0 2^-8 + p1 2^-24 + p2 2^-40 + p3 2^-56 to the nearest 2^-42, the size of the
-        // operands' own rounding; |p0| < 2^28 + 2^23, so below 2^63
-        const long long n = static_cast<long long>(p[t][0]) * (1ll << 34) + static_cast<long long>(p[t][1]) * (1 << 18) +
-                            static_cast<long long>(p[t][2]) * 4 + ((p[t][3] >> 14) + ((p[t][3] >> 13) & 1));
-        double v = rounded(n, static_cast<int>(el + er[t]) - 2044 - 56);
-        if (el == 0x7ffu || er[t] == 0x7ffu) v = __longlong_as_double(0x7ff8000000000000ll);
-        if constexpr (kMode == kScale) {
-          if (!first) v += sm.part[k][threadIdx.x];
-          if (last) acc[k] = fma(alpha, v, acc[k]);
-          else sm.part[k][threadIdx.x] = v;
-        } else if constexpr (kMode == kAdd) {
-          acc[k] += v;
+        const double v = value(p[t][0], p[t][1], p[t][2], p[t][3], el, er[t]);
+        if constexpr (kEach) {
+          if (c0 + q + t < S.x.cols) *to = v;
+          to += S.x.lds;
         } else {
-          acc[k] = v;
+          acc[q + t] = fma(S.x.alpha, v, acc[q + t]);
         }
       }
     }
   }
-  template <Mode kMode>
-  __device__ __forceinline__ void finish_any(int rows, int cols, bool first, bool last) {
-    if (rows > 32) finish<8, kMode>(rows, cols, first, last);
-    else finish<4, kMode>(rows, cols, first, last);
+
+  // Of the staged step, the outputs (bits) of this thread that have a product near that of the
+  // scales, and << 8 those that have one that is not zero.
+  template <int kOut>
+  __device__ __forceinline__ unsigned int weigh(int cols) const {
+    if (col_of(kOut == 8) >= cols) return 0u;
+    const uint4 l = sm.weight[row_of(kOut == 8)], *w = sm.weight + kDgRows + col_of(kOut == 8);
+    unsigned int f = 0u;
+#pragma unroll
+    for (int k = 0; k < kOut; k++) {
+      const unsigned int hit = (l.x & w[k].x) | (l.y & w[k].y) | (l.z & w[k].z) | (l.w & w[k].w);
+      if (hit > 255u) f |= 1u << k;
+      if (hit != 0u) f |= 256u << k;
+    }
+    return f;
+  }
+  // The same of any step, one output after another: a product's steps are added up in sm.part,
+  // so that an item is rounded into acc once whatever its inner dimension, as on the FP64
+  // pipe. f: the outputs that are formed by multiply-adds.
+  template <bool kEach>
+  __device__ __forceinline__ void finish_part(const DgStep& S, unsigned int f) {
+    const bool big = S.x.rows > 32;
+    const int r = row_of(big), c0 = col_of(big), n = min(big ? 8 : 4, S.x.cols - c0);
+    const int* s = sm.sums + r * kDgSumLd + c0;
+    const unsigned int* expo = sm.expo[held];
+#pragma unroll 1
+    for (int k = 0; k < n; k++) {
+      double v;
+      if (f >> k & 1u)
+        v = dg_direct(S, r, c0 + k);
+      else
+        v = value(s[k], s[k + kDgRows * kDgSumLd], s[k + 2 * kDgRows * kDgSumLd], s[k + 3 * kDgRows * kDgSumLd],
+                  expo[r], expo[kDgRows + c0 + k]);
+      if (!S.first) v += sm.part[k][threadIdx.x];
+      if (kEach && S.last) S.x.s[r + static_cast<int64_t>(S.x.lds) * (c0 + k)] = v;
+      else sm.part[k][threadIdx.x] = v;
+    }
+    if (!kEach && S.last) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k < n) acc[k] = fma(S.x.alpha, sm.part[k][threadIdx.x], acc[k]);
+    }
+  }
+
+  // A step's sums (collected), `weighed` by weigh.
+  template <bool kEach>
+  __device__ __forceinline__ void finish(unsigned int weighed) {
+    const DgStep& S = sm.step[at];
+    const bool big = S.x.rows > 32;
+    const int r = row_of(big), c0 = col_of(big);
+    if (r >= S.x.rows || c0 >= S.x.cols) return;
+    const unsigned int f = weighed >> 8 & ~weighed & ((1u << min(S.x.cols - c0, 8)) - 1u);
+    if (!S.first || !S.last) {
+      finish_part<kEach>(S, f);
+      return;
+    }
+    // the outputs that are formed by multiply-adds: zeros for their sums, and themselves afterwards
+    for (unsigned int g = f; g != 0u; g &= g - 1u)
+#pragma unroll
+      for (int c = 0; c < kDgDiagonals / 2; c++)
+        sm.sums[(c * kDgRows + r) * kDgSumLd + c0 + __ffs(static_cast<int>(g)) - 1] = 0;
+    if (big) finish_whole<8, kEach>(S);
+    else finish_whole<4, kEach>(S);
+    if (f == 0u) return;
+    for (unsigned int g = f; g != 0u; g &= g - 1u) {
+      const int k = __ffs(static_cast<int>(g)) - 1;
+      const double v = dg_direct(S, r, c0 + k);
+      if constexpr (kEach) S.x.s[r + static_cast<int64_t>(S.x.lds) * (c0 + k)] = v;
+      else sm.part[k][threadIdx.x] = v;
+    }
+    if constexpr (!kEach) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (f >> k & 1u) acc[k] = fma(S.x.alpha, sm.part[k][threadIdx.x], acc[k]);
+    }
   }
 };
 
 // Streams the products of sm.rec through the engine. Src: count(); prepare(q), called by all
-// threads before record q is read (it may refill sm.rec and hold barriers), returns its slot;
-// store(), called when a product's sums are complete (kEach: after every product; else the
-// sums of all products add up and stay in the engine).
+// threads before record q is read (it may refill sm.rec and hold barriers), returns its slot.
+// kEach: every product goes to its place in memory; else the sums of all add up in the engine.
 template <bool kEach, class Src>
 __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
   DgSmem& sm = E.sm;
@@ -394,27 +516,23 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     dg_load(u, is_l ? X.l : X.r, is_l ? X.lld : X.rld, is_l ? X.ltrans : X.rtrans, row, k0 + 8 * kg, rem - 8 * kg);
     return row | kg << 8 | (is_l ? 1 << 12 : 0) | 1 << 13;
   };
-  auto cut = [&](const DgUnit& u, int w, const unsigned int* expo) {
+  auto cut = [&](const DgUnit& u, int w, const unsigned int* expo, bool short_k) {
     if (!(w & (1 << 13))) return;
     const int row = w & 0xff, kg = (w >> 8) & 0xf;
-    if (w & (1 << 12)) dg_store<kDgRows>(u, expo[row], sm.l, kDgLBytes, row, kg);
-    else dg_store<kDgCols>(u, expo[kDgRows + row], sm.r, kDgRBytes, row, kg);
-  };
-
-  // the previous step's product: its extents, and in pass 1 where it goes and whether complete
-  int prows = 0, pcols = 0, plds = 0;
-  double* ps = nullptr;
-  bool pfirst = false, plast = false;
-  auto complete = [&]() {
-    if constexpr (kEach) {
-      if (pfirst) E.template finish_any<DgEngine::kSet>(prows, pcols, true, true);
-      else E.template finish_any<DgEngine::kAdd>(prows, pcols, true, true);
-      if (plast) src.store(E, ps, plds, prows, pcols);
+    if (w & (1 << 12)) {
+      dg_store<kDgRows>(u, expo[row], sm.l, kDgLBytes, row, kg);
+      uint32_t* weight = reinterpret_cast<uint32_t*>(&sm.weight[row]);
+      weight[kg] = dg_weight(u, expo[row]);
+      if (short_k) weight[kg + 2] = 0u;
     } else {
-      E.template finish_any<DgEngine::kScale>(prows, pcols, pfirst, plast);
+      dg_store<kDgCols>(u, expo[kDgRows + row], sm.r, kDgRBytes, row, kg);
+      // the classes in reverse, so that d <= 1, 3, 5 of L meet d <= 5, 3, 1 of R
+      reinterpret_cast<uint32_t*>(&sm.weight[kDgRows + row])[kg] =
+          __byte_perm(dg_weight(u, expo[kDgRows + row]), 0u, 0x1230);
     }
   };
 
+  unsigned int pweighed = 0u;  // of the step in flight
   seek();
   if (more) {
     w0 = fetch(u0, utid);
@@ -436,11 +554,12 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     if (k0 == kDgK && E.flying) onto = !__syncthreads_or(tid < kDgRows + kDgCols && expo[tid] > before[tid]);
     if (E.flying) {
       E.wait();
-      if (!onto) E.collect(prows, pcols);
+      if (!onto) E.collect();
     }
-    // the digits (the MMAs that read the buffers are done)
-    cut(u0, w0, onto ? before : expo);
-    cut(u1, w1, onto ? before : expo);
+    // the digits (the MMAs that read the buffers are done) and weights
+    const bool short_k = sm.rec[slot].k - k0 <= 16;
+    cut(u0, w0, onto ? before : expo, short_k);
+    cut(u1, w1, onto ? before : expo, short_k);
     fence_async_smem();
     if (__syncthreads_or(!E.ok)) return false;
     const DgRecord& X = sm.rec[slot];
@@ -449,10 +568,19 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
       if (elect_one()) E.issue(rem > 16 ? 2 : 1, onto);
       __syncwarp();
     }
-    const double alpha = X.alpha;
-    const int rows = X.rows, cols = X.cols, lds = X.lds;
-    double* const s = X.s;
+    const int rows = X.rows, cols = X.cols;
     const bool first = k0 == 0, last = rem <= kDgK;
+    const unsigned int weighed = rows > 32 ? E.template weigh<8>(cols) : E.template weigh<4>(cols);
+    if (tid == 0) {
+      DgStep& S = sm.step[onto ? E.at : E.at ^ 1];
+      S.k1 = k0 + min(rem, kDgK);
+      S.last = last;
+      if (!onto) {
+        S.x = X;
+        S.k0 = k0;
+        S.first = first;
+      }
+    }
     // the next step's operands; an operand that this step staged as well is not read again
     same_l = same_r = false;
     if (!last) {
@@ -472,24 +600,21 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
       w0 = fetch(u0, utid);
       w1 = fetch(u1, utid + kDgThreads);
     }
-    if (E.flying && !onto) complete();
+    if (E.flying && !onto) E.template finish<kEach>(pweighed);
     E.flying = true;
-    E.alpha = alpha;
-    if (!onto) E.held = E.cur;
+    if (!onto) {
+      E.held = E.cur;
+      E.at ^= 1;
+    }
     E.cur = spare;
-    prows = rows;
-    pcols = cols;
-    plds = lds;
-    ps = s;
-    pfirst = first || (onto && pfirst);
-    plast = last;
+    pweighed = onto ? pweighed | weighed : weighed;
   }
   if (E.flying) {
     __syncthreads();  // the last sums have been read
     E.wait();
-    E.collect(prows, pcols);
+    E.collect();
     if (__syncthreads_or(!E.ok)) return false;
-    complete();
+    E.template finish<kEach>(pweighed);
     E.flying = false;
   }
   return true;
@@ -500,14 +625,6 @@ struct DgInterSource {
   int units;
   __device__ __forceinline__ int count() const { return units; }
   __device__ __forceinline__ int prepare(int q) const { return q; }
-  __device__ __forceinline__ void store(const DgEngine& E, double* s, int lds, int rows, int cols) const {
-    const bool big = rows > 32;
-    const int r = DgEngine::row_of(big), c0 = DgEngine::col_of(big);
-    if (r >= rows) return;
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (k < (big ? 8 : 4) && c0 + k < cols) s[r + static_cast<int64_t>(lds) * (c0 + k)] = E.acc[k];
-  }
 };
 
 // Pass 2: the items of a tile half, their records made from the item list kDgBatch at a time.
@@ -554,10 +671,6 @@ __device__ void dg_setup(DgSmem& sm) {
   }
   for (int i = threadIdx.x; i < 3 * (kDgRows + kDgCols); i += kDgThreads)
     sm.expo[i / (kDgRows + kDgCols)][i % (kDgRows + kDgCols)] = 0u;
-  // the digit of zeros of either half of R's K
-  constexpr int kZero = kDgCols * kDgRowBytes;
-  for (int i = threadIdx.x; i < 2 * kZero / 4; i += kDgThreads)
-    *reinterpret_cast<uint32_t*>(sm.r + (i / (kZero / 4)) * kDgRBytes + kDgDigits * kZero + 4 * (i % (kZero / 4))) = 0u;
   fence_async_smem();
   if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
@@ -717,7 +830,6 @@ __global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
 }
 
 constexpr int kDgSmemBytes = static_cast<int>(sizeof(DgSmem)) + 1024;
-constexpr int kDgInterBytes = static_cast<int>(offsetof(DgSmem, part)) + 1024;  // what pass 1 uses of it
 
 int dg_grid(int units) {
   static const int sms = [] {
@@ -736,12 +848,12 @@ cudaError_t launch_inter_digits(const InterJob* jobs, const GemmTile* tiles, int
                                 unsigned int* sched, int* err, cudaStream_t stream) {
   if (ntiles <= 0) return cudaSuccess;
   const cudaError_t e =
-      cudaFuncSetAttribute(inter_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgInterBytes);
+      cudaFuncSetAttribute(inter_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
   if (e != cudaSuccess) return e;
   const int grid = dg_grid(ntiles);
   // several batches a CTA, so that no CTA is left with a long one at the end
   const int take = std::max(1, std::min(kDgBatch / 2, ntiles / (4 * grid)));
-  inter_digits_kernel<<<grid, kDgThreads, kDgInterBytes, stream>>>(jobs, tiles, ntiles, take, sp, sched, err);
+  inter_digits_kernel<<<grid, kDgThreads, kDgSmemBytes, stream>>>(jobs, tiles, ntiles, take, sp, sched, err);
   return cudaGetLastError();
 }
 

@@ -251,6 +251,13 @@ int c2g_truncation_eig(int count, const int* n, const double* mats, double* eval
  * leading (n-1) x (n-1) block, as in a Davidson expansion step. */
 int c2g_rayleigh_ritz_eig(int n, const double* mat, int warm, double* evals, double* evecs, int reps,
                           double* us_per_call);
+/* The FP64 products of the two-pass path, exposed for testing: products[i] = L_i R_i and
+ * sum = sum_i alpha_i L_i R_i (added over `splits` ranges of i) for `count` pairs of blocks, m x k and
+ * k x n, column-major and concatenated; trans & 1: the L_i are stored transposed, trans & 2:
+ * the R_i. digits != 0: on the tensor cores (as exact products of digits); 0: on the FP64
+ * pipe. All sizes at most 4096. */
+int c2g_two_pass_products(int digits, int m, int n, int k, int count, int trans, int splits, const double* l,
+                          const double* r, const double* alpha, double* products, double* sum);
 /* No counterpart in the reference (a diagnostic): the free memory of `device` (< 0: the
  * calling thread's current device; cudaMemGetInfo) and the bytes in use from that
  * device's default stream-ordered pool (cudaMemPoolAttrUsedMemCurrent), where this
