@@ -49,8 +49,8 @@
 //
 // Every mbarrier wait is bounded: after kTcSpinLimit polls the kernel records an error in
 // the runtime's mapped error word, frees its tensor memory and returns without writing its
-// tile. An infinite or NaN element makes its row's or column's outputs NaN; elements below the
-// normal range count as zero.
+// tile. A step with an infinite or NaN element is formed by multiply-adds as a whole;
+// elements below the normal range count as zero in the others.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -356,10 +356,8 @@ struct DgEngine {
 
   // The value of diagonals p in units of 2^e / 2^2044: p0 2^-20 + p1 2^-36 + p2 2^-52 + p3 2^-68
   __device__ __forceinline__ static double value(int p0, int p1, int p2, int p3, unsigned int el, unsigned int er) {
-    double v = rounded(static_cast<long long>(p0) * 65536 + p1, static_cast<long long>(p2) * 65536 + p3,
-                       static_cast<int>(el + er) - 2044 - 68);
-    if (el == 0x7ffu || er == 0x7ffu) v = __longlong_as_double(0x7ff8000000000000ll);
-    return v;
+    return rounded(static_cast<long long>(p0) * 65536 + p1, static_cast<long long>(p2) * 65536 + p3,
+                   static_cast<int>(el + er) - 2044 - 68);
   }
 
   // The collected sums of a whole product, each rounded once: to memory, or times alpha into acc.
@@ -396,6 +394,7 @@ struct DgEngine {
     }
   }
 
+  static constexpr unsigned int kAllDirect = 1u << 16;  // all outputs of a step by multiply-adds
   // Of the staged step, the outputs (bits) of this thread that have a product near that of the
   // scales, and << 8 those that have one that is not zero.
   template <int kOut>
@@ -439,14 +438,15 @@ struct DgEngine {
     }
   }
 
-  // A step's sums (collected), `weighed` by weigh.
+  // A step's sums (collected), `weighed` by weigh or kAllDirect.
   template <bool kEach>
   __device__ __forceinline__ void finish(unsigned int weighed) {
     const DgStep& S = sm.step[at];
     const bool big = S.x.rows > 32;
     const int r = row_of(big), c0 = col_of(big);
     if (r >= S.x.rows || c0 >= S.x.cols) return;
-    const unsigned int f = weighed >> 8 & ~weighed & ((1u << min(S.x.cols - c0, 8)) - 1u);
+    const unsigned int f = (weighed >= kAllDirect ? 255u : weighed >> 8 & ~weighed) &
+                           ((1u << min(S.x.cols - c0, big ? 8 : 4)) - 1u);
     if (!S.first || !S.last) {
       finish_part<kEach>(S, f);
       return;
@@ -547,7 +547,11 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     if (tid < kDgRows + kDgCols && (tid < kDgRows ? same_l : same_r)) expo[tid] = before[tid];
     __syncthreads();
     const int spare = 3 - E.held - E.cur;  // last read a step ago
-    if (tid < kDgRows + kDgCols) sm.expo[spare][tid] = 0u;
+    bool odd = false;  // an infinite or NaN element
+    if (tid < kDgRows + kDgCols) {
+      sm.expo[spare][tid] = 0u;
+      odd = expo[tid] == 0x7ffu;
+    }
     // The second 32 of K go onto the first ones' sums where their scales will do: the sums of
     // 64 products of a diagonal are exact as well, and pairs of them below 2^31.
     bool onto = false;
@@ -561,7 +565,8 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     cut(u0, w0, onto ? before : expo, short_k);
     cut(u1, w1, onto ? before : expo, short_k);
     fence_async_smem();
-    if (__syncthreads_or(!E.ok)) return false;
+    odd = __syncthreads_or(!E.ok || odd);
+    if (odd && __syncthreads_or(!E.ok)) return false;
     const DgRecord& X = sm.rec[slot];
     const int rem = X.k - k0;
     if (warp == kDgIssuer) {
@@ -570,7 +575,9 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     }
     const int rows = X.rows, cols = X.cols;
     const bool first = k0 == 0, last = rem <= kDgK;
-    const unsigned int weighed = rows > 32 ? E.template weigh<8>(cols) : E.template weigh<4>(cols);
+    const unsigned int weighed = odd         ? DgEngine::kAllDirect
+                                 : rows > 32 ? E.template weigh<8>(cols)
+                                             : E.template weigh<4>(cols);
     if (tid == 0) {
       DgStep& S = sm.step[onto ? E.at : E.at ^ 1];
       S.k1 = k0 + min(rem, kDgK);

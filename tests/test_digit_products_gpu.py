@@ -76,3 +76,26 @@ def test_each_element_is_as_accurate_as_multiply_adds(kind):
         print(f"{kind} {m} x {k} x {n}: rms error over sum |l||r|, in u: digits {rms[0]:.2f}, FP64 pipe {rms[1]:.2f}")
     d, p = np.mean(worst, axis=0)
     assert d <= 1.25 * p  # no less accurate than the multiply-adds that the path replaces
+
+
+def test_infinite_and_nan_elements_as_multiply_adds_give_them():
+    rng = np.random.default_rng(5)
+    for m, n, k in [(17, 20, 12), (40, 33, 32), (47, 47, 47)]:
+        l, r = rng.standard_normal((3, m, k)), rng.standard_normal((3, k, n))
+        l[0, 3, 5], l[0, 4, 0], r[0, k - 1, 7] = np.inf, -np.inf, np.inf
+        l[0, :, 2] = 0.0
+        r[0, 5, 9] = 0.0  # infinity times zero
+        r[0, 2, 11] = -np.inf  # every row of L is zero there
+        r[0, :, 1] = 0.0
+        l[1, m - 1, k - 1] = np.nan
+        r[1, :, 4] = 0.0
+        with np.errstate(invalid="ignore"):
+            ref = np.einsum("imk,ikn->imn", l, r, optimize=False)
+            terms = l[:, :, :, None] * r[:, None, :, :]
+            total = terms.sum(axis=2)
+        for trans in (0, 3):
+            p, _ = products(l, r, np.ones(3), trans)
+            assert np.array_equal(np.isnan(p), np.isnan(total)), (m, n, k)
+            assert np.array_equal(np.isinf(p), np.isinf(ref)) and np.all(p[np.isinf(p)] == ref[np.isinf(p)]), (m, n, k)
+            ok = np.isfinite(ref)
+            assert np.all(np.abs(p[ok] - ref[ok]) <= (8 * k + 4) * U * np.abs(terms).sum(axis=2)[ok]), (m, n, k)
