@@ -49,8 +49,8 @@
 //
 // Every mbarrier wait is bounded: after kTcSpinLimit polls the kernel records an error in
 // the runtime's mapped error word, frees its tensor memory and returns without writing its
-// tile. A step with an infinite or NaN element is formed by multiply-adds as a whole;
-// elements below the normal range count as zero in the others.
+// tile. A step with an infinite or NaN element, or with a scale that may take a result out of
+// the normal range, is formed by multiply-adds as a whole.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -72,6 +72,11 @@ constexpr int kDgDigits = 8, kDgDiagonals = kDgDigits;
 constexpr int kDgRows = 64, kDgCols = 32, kDgK = 32;  // of a step
 constexpr uint32_t kDgTmemCols = kDgDiagonals * kDgCols;
 constexpr int kDgBatch = 32;                          // records held in shared memory
+
+// Exponent fields of the scales that digits take: those of a row and a column add up to at least
+// 1092 and at most 3060, so that every sum, a multiple of 2^-68 of the scales' product and at most
+// 2^6 times that, is a normal number.
+constexpr unsigned int kDgExpoMin = 546, kDgExpoMax = 1530;
 
 // K-major rows without swizzle, 16 of K at a time: 8-row groups of 256 bytes, 128 bytes
 // between the two 8-wide halves of K
@@ -170,6 +175,7 @@ __device__ __forceinline__ unsigned long long dg_fixed(double v, unsigned int em
 // of byte 3 where d <= 1.
 __device__ __forceinline__ uint32_t dg_weight(const DgUnit& u, unsigned int emax) {
   uint32_t w = 0u;
+  emax = max(emax, 6u);  // in a row of subnormal elements all are far below it
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     const unsigned int hi = __double2hiint(u.v[k]), lo = __double2loint(u.v[k]);
@@ -214,8 +220,8 @@ __device__ __forceinline__ void dg_store(const DgUnit& u, unsigned int emax, uns
 }
 
 // (hi 2^32 + lo) 2^k as a double to the nearest, by the bits (a conversion or an FP64
-// instruction costs a warp 65 clocks); |hi| < 2^62, |lo| < 2^62. A negative one is off by a unit
-// of lo before it is rounded. Zero where the result is below the normal range, infinite above it.
+// instruction costs a warp 65 clocks); |hi| < 2^62, |lo| < 2^62, the result in the normal
+// range. A negative one is off by a unit of lo before it is rounded.
 __device__ __forceinline__ double rounded(long long hi, long long lo, int k) {
   hi += lo >> 32;
   const unsigned int s = static_cast<unsigned int>(hi >> 63);
@@ -231,9 +237,7 @@ __device__ __forceinline__ double rounded(long long hi, long long lo, int k) {
   const unsigned long long m = (u >> 11) + ((u >> 10) & 1u);  // 2^52 .. 2^53
   const unsigned long long v = (static_cast<unsigned long long>(f - 1) << 52) + m;
   const unsigned int top = static_cast<unsigned int>(v >> 32) | (s & 0x80000000u);
-  if (w2 == 0u || f <= 0) return 0.0;
-  if (f >= 0x7fe) return __hiloint2double((s & 0x80000000u) | 0x7ff00000u, 0);
-  return __hiloint2double(top, static_cast<unsigned int>(v));
+  return w2 == 0u ? 0.0 : __hiloint2double(top, static_cast<unsigned int>(v));
 }
 
 // Output (i, j) of a step by FP64 multiply-adds.
@@ -547,10 +551,11 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     if (tid < kDgRows + kDgCols && (tid < kDgRows ? same_l : same_r)) expo[tid] = before[tid];
     __syncthreads();
     const int spare = 3 - E.held - E.cur;  // last read a step ago
-    bool odd = false;  // an infinite or NaN element
+    bool odd = false;  // a scale so small or large that a result may leave the normal range, an infinity or a NaN
     if (tid < kDgRows + kDgCols) {
       sm.expo[spare][tid] = 0u;
-      odd = expo[tid] == 0x7ffu;
+      const unsigned int x = expo[tid];
+      odd = x != 0u && x - kDgExpoMin > kDgExpoMax - kDgExpoMin;
     }
     // The second 32 of K go onto the first ones' sums where their scales will do: the sums of
     // 64 products of a diagonal are exact as well, and pairs of them below 2^31.

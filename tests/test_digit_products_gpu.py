@@ -99,3 +99,33 @@ def test_infinite_and_nan_elements_as_multiply_adds_give_them():
             assert np.array_equal(np.isinf(p), np.isinf(ref)) and np.all(p[np.isinf(p)] == ref[np.isinf(p)]), (m, n, k)
             ok = np.isfinite(ref)
             assert np.all(np.abs(p[ok] - ref[ok]) <= (8 * k + 4) * U * np.abs(terms).sum(axis=2)[ok]), (m, n, k)
+
+
+def test_ends_of_the_range_are_those_of_multiply_adds():
+    """Blocks whose scales or results are near either end of the range: the digits leave them to
+    the same multiply-adds, in the same order, as the FP64 pipe, so the results are equal."""
+    rng = np.random.default_rng(6)
+    for m, n, k in [(17, 20, 12), (40, 33, 32), (33, 17, 20)]:
+        l, r = rng.standard_normal((6, m, k)), rng.standard_normal((6, k, n))
+        l[0] *= 2.0**-1040  # subnormal
+        r[0] *= 2.0**40
+        l[1, 2] *= 2.0**-900  # products below the normal range
+        r[1] *= 2.0**-140
+        l[2] *= 2.0**600  # sums of up to 2^1024
+        r[2] *= 2.0**420
+        l[3, :, 1:] = 0.0  # one product of 2^1023 to 2^1024
+        l[3, :, 0], r[3, 0] = 1.25 * 2.0**500, 1.25 * 2.0**523
+        r[4, :, 3] = 0.0
+        r[4, 7, 3] = 5e-324  # the only element of its column
+        l[5, :, :] = rng.standard_normal((m, k)) * 2.0**-1074
+        l[5, 1] = 0.0
+        with np.errstate(over="ignore"):
+            p, _ = products(l, r, np.ones(6))
+            q, _ = products(l, r, np.ones(6), digits=0)
+        assert np.array_equal(p[[0, 1, 2, 3, 5]], q[[0, 1, 2, 3, 5]], equal_nan=True), (m, n, k)
+        assert np.array_equal(p[4, :, 3], q[4, :, 3]), (m, n, k)
+        assert np.isfinite(q[3]).all() and np.any(q[4, :, 3] != 0.0)
+    l, r = rng.standard_normal((1, 17, 12)) * 2.0**600, rng.standard_normal((1, 12, 20)) * 2.0**424
+    p, _ = products(l, r, [1.0])
+    q, _ = products(l, r, [1.0], digits=0)
+    assert np.isinf(q).any() and np.isfinite(q).any() and np.array_equal(p, q, equal_nan=True)
