@@ -783,7 +783,7 @@ int c2g_rayleigh_ritz_eig(int n, const double* mat, int warm, double* evals, dou
 }
 
 int c2g_two_pass_products(int digits, int m, int n, int k, int count, int trans, int splits, const double* l,
-                          const double* r, const double* alpha, double* products, double* sum) {
+                          const double* r, const double* alpha, double* products, double* sum, double* given_up) {
   return guarded([&] {
     if (m < 1 || n < 1 || k < 1 || m > 4096 || n > 4096 || k > 4096 || count < 1 || count > 4096 || splits < 1 ||
         splits > count || trans < 0 || trans > 3)
@@ -857,17 +857,25 @@ int c2g_two_pass_products(int digits, int m, int n, int k, int count, int trans,
     auto* words = static_cast<unsigned*>(put(nullptr, 4 * (5 + stiles.size())));  // scheduler, error, counters
     int* err = reinterpret_cast<int*>(words + 4);
     const int nj = static_cast<int>(jtiles.size()), ns = static_cast<int>(stiles.size());
-    if (digits) {
-      C2G_CUDA(c2g::launch_inter_digits(dj, djt, nj, sp, words, err, nullptr));
-      C2G_CUDA(c2g::launch_sum_digits(dg, di, dst, ns, part, words + 5, sp, words + 2, err, nullptr));
-    } else {
-      C2G_CUDA(c2g::launch_inter_gemm(dj, djt, nj, sp, nullptr, c2g::Precision::kFP64));
-      C2G_CUDA(c2g::launch_sum_gemm(dg, di, dst, ns, part, words + 5, sp, nullptr, c2g::Precision::kFP64));
-    }
-    C2G_CUDA(cudaMemcpy(products, sp.inter, 8 * mp * count, cudaMemcpyDeviceToHost));
-    C2G_CUDA(cudaMemcpy(sum, sp.y, 8 * mp, cudaMemcpyDeviceToHost));
     int e = 0;
-    C2G_CUDA(cudaMemcpy(&e, err, sizeof(e), cudaMemcpyDeviceToHost));
+    auto run = [&](double* products_to, double* sum_to, bool give_up) {
+      if (digits) {
+        C2G_CUDA(c2g::launch_inter_digits(dj, djt, nj, sp, words, err, nullptr, give_up));
+        C2G_CUDA(c2g::launch_sum_digits(dg, di, dst, ns, part, words + 5, sp, words + 2, err, nullptr, give_up));
+      } else {
+        C2G_CUDA(c2g::launch_inter_gemm(dj, djt, nj, sp, nullptr, c2g::Precision::kFP64));
+        C2G_CUDA(c2g::launch_sum_gemm(dg, di, dst, ns, part, words + 5, sp, nullptr, c2g::Precision::kFP64));
+      }
+      C2G_CUDA(cudaMemcpy(products_to, sp.inter, 8 * mp * count, cudaMemcpyDeviceToHost));
+      C2G_CUDA(cudaMemcpy(sum_to, sp.y, 8 * mp, cudaMemcpyDeviceToHost));
+      C2G_CUDA(cudaMemcpy(&e, err, sizeof(e), cudaMemcpyDeviceToHost));
+    };
+    if (given_up && digits) {
+      run(given_up, given_up + mp * count, true);
+      if (e == 0) throw std::logic_error("c2g_two_pass_products: no wait was given up");
+      C2G_CUDA(cudaMemset(err, 0, sizeof(e)));
+    }
+    run(products, sum, false);
     if (e) throw std::runtime_error("c2g_two_pass_products: a kernel gave up a wait");
   });
 }

@@ -137,12 +137,13 @@ cudaError_t launch_sum_tc(const SumGroup* groups, const SumItem* items, const Ge
                           cudaStream_t stream);
 
 // The two passes in FP64 on the tensor cores, as exact products of digits
-// (sandwich_digits.cu); `sched` and `err` as above.
+// (sandwich_digits.cu); `sched` and `err` as above. A kernel that gives up a wait sets the error
+// word and writes NaN; give_up: it gives up every wait (for tests).
 cudaError_t launch_inter_digits(const InterJob* jobs, const GemmTile* tiles, int ntiles, const SlotPtrs& sp,
-                                unsigned int* sched, int* err, cudaStream_t stream);
+                                unsigned int* sched, int* err, cudaStream_t stream, bool give_up = false);
 cudaError_t launch_sum_digits(const SumGroup* groups, const SumItem* items, const GemmTile* tiles, int ntiles,
                               double* partials, unsigned int* counters, const SlotPtrs& sp, unsigned int* sched,
-                              int* err, cudaStream_t stream);
+                              int* err, cudaStream_t stream, bool give_up = false);
 
 cudaError_t launch_sandwich(const Group* groups, const Term* terms, const BatchEntry* entries, const TileDesc* tiles,
                             int ntiles, const SlotPtrs& sp, cudaStream_t stream, Precision prec = Precision::kFP64);

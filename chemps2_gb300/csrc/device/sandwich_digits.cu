@@ -47,11 +47,13 @@
 // 3.0 / 4.4, 9.1 / 10.6 and 12.2 / 13.7, but outputs without a product near M lost up to all of their
 // digits. Below about 17 x 17 x 12 the FP64 pipe is the faster one (digits_pay in runtime.cpp).
 //
-// Every mbarrier wait is bounded: after kTcSpinLimit polls the kernel records an error in
-// the runtime's mapped error word, frees its tensor memory and returns without writing its
-// tile. A step with an infinite or NaN element, or with a scale that may take a result out of
+// Every mbarrier wait is bounded: after kPolls polls a CTA records an error in the runtime's
+// mapped error word, writes NaN to that tile and to all that it takes after it (so that split
+// tiles still meet at their counters), and frees its tensor memory once its MMAs are done, or
+// after a second bounded wait. A step with an infinite or NaN element, or with a scale that may take a result out of
 // the normal range, is formed by multiply-adds as a whole.
 #include <cuda_fp16.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <cstddef>
@@ -287,6 +289,8 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[16]) {
 }
 
 // The running state of a CTA: the step in flight on the tensor cores and the sums so far.
+// kPolls: of a wait.
+template <long long kPolls>
 struct DgEngine {
   DgSmem& sm;
   uint32_t tmem;
@@ -325,10 +329,14 @@ struct DgEngine {
   }
 
   __device__ __forceinline__ void wait() {
-    if (!mbar_wait(&sm.bar, phase)) ok = false;
+    if (!mbar_wait(&sm.bar, phase, kPolls)) ok = false;
     phase ^= 1u;
     tc_fence_after();
   }
+
+  // False where the MMAs may still be running, but not asked after a wait of kTcSpinLimit polls:
+  // what follows is not used then.
+  __device__ __forceinline__ bool live() const { return kPolls > 0 || ok; }
 
   // Tensor memory -> shared memory: warp w holds rows 32 (w % 4) .. + 31 and columns
   // 16 (w / 4) .. + 15. Two diagonals make one integer, 256 i_c + i_(c+1), below 2^31.
@@ -480,8 +488,8 @@ struct DgEngine {
 // Streams the products of sm.rec through the engine. Src: count(); prepare(q), called by all
 // threads before record q is read (it may refill sm.rec and hold barriers), returns its slot.
 // kEach: every product goes to its place in memory; else the sums of all add up in the engine.
-template <bool kEach, class Src>
-__device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
+template <bool kEach, long long kPolls, class Src>
+__device__ __forceinline__ bool dg_stream(DgEngine<kPolls>& E, Src& src) {
   DgSmem& sm = E.sm;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -563,12 +571,14 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     if (k0 == kDgK && E.flying) onto = !__syncthreads_or(tid < kDgRows + kDgCols && expo[tid] > before[tid]);
     if (E.flying) {
       E.wait();
-      if (!onto) E.collect();
+      if (!onto && E.live()) E.collect();
     }
     // the digits (the MMAs that read the buffers are done) and weights
-    const bool short_k = sm.rec[slot].k - k0 <= 16;
-    cut(u0, w0, onto ? before : expo, short_k);
-    cut(u1, w1, onto ? before : expo, short_k);
+    if (E.live()) {
+      const bool short_k = sm.rec[slot].k - k0 <= 16;
+      cut(u0, w0, onto ? before : expo, short_k);
+      cut(u1, w1, onto ? before : expo, short_k);
+    }
     fence_async_smem();
     odd = __syncthreads_or(!E.ok || odd);
     if (odd && __syncthreads_or(!E.ok)) return false;
@@ -580,7 +590,7 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
     }
     const int rows = X.rows, cols = X.cols;
     const bool first = k0 == 0, last = rem <= kDgK;
-    const unsigned int weighed = odd         ? DgEngine::kAllDirect
+    const unsigned int weighed = odd         ? E.kAllDirect
                                  : rows > 32 ? E.template weigh<8>(cols)
                                              : E.template weigh<4>(cols);
     if (tid == 0) {
@@ -624,7 +634,7 @@ __device__ __forceinline__ bool dg_stream(DgEngine& E, Src& src) {
   if (E.flying) {
     __syncthreads();  // the last sums have been read
     E.wait();
-    E.collect();
+    if (E.live()) E.collect();
     if (__syncthreads_or(!E.ok)) return false;
     E.template finish<kEach>(pweighed);
     E.flying = false;
@@ -712,7 +722,8 @@ __device__ __forceinline__ int dg_next(unsigned int* sched, int* slot, int take)
   return *slot;
 }
 
-__device__ __forceinline__ void dg_end(DgEngine& E, unsigned int* sched, int* err) {
+template <long long kPolls>
+__device__ __forceinline__ void dg_end(DgEngine<kPolls>& E, unsigned int* sched, int* err) {
   if (__syncthreads_or(!E.ok)) {
     if (threadIdx.x == 0 && err) atomicOr(err, 2);
     mbar_wait(&E.sm.bar, E.phase ^ 1u);  // the MMAs still in flight, bounded again
@@ -725,48 +736,110 @@ __device__ __forceinline__ void dg_end(DgEngine& E, unsigned int* sched, int* er
   dg_teardown(E.tmem);
 }
 
+// The records of pass 1's job tiles first .. first + n - 1, the two column halves of each.
+__device__ __forceinline__ void dg_inter_batch(DgSmem& sm, const InterJob* __restrict__ jobs,
+                                               const GemmTile* __restrict__ tiles, int first, int n,
+                                               const SlotPtrs& sp) {
+  if (static_cast<int>(threadIdx.x) < 2 * n) {
+    const GemmTile T = tiles[first + (threadIdx.x >> 1)];
+    const InterJob J = jobs[T.idx];
+    const int row0 = (T.pos >> 16) * 64, col0 = (T.pos & 0xffff) * 64 + (threadIdx.x & 1) * kDgCols;
+    DgRecord d{};
+    d.rows = static_cast<int16_t>(min(64, J.m - row0));
+    d.cols = static_cast<int16_t>(min(kDgCols, J.n - col0));
+    d.k = d.cols > 0 ? J.k : 0;
+    if (d.cols > 0) {
+      d.l = resolve<double>(sp, J.l.ref) + (J.l.trans ? static_cast<int64_t>(J.l.ld) * row0 : row0);
+      d.r = resolve<double>(sp, J.r.ref) + (J.r.trans ? col0 : static_cast<int64_t>(J.r.ld) * col0);
+      d.s = sp.inter + J.off + row0 + static_cast<int64_t>(J.m) * col0;
+    }
+    d.alpha = 1.0;
+    d.lld = J.l.ld;
+    d.rld = J.r.ld;
+    d.lds = J.m;
+    d.ltrans = J.l.trans != 0;
+    d.rtrans = J.r.trans == 0;
+    sm.rec[threadIdx.x] = d;
+  }
+  __syncthreads();
+}
+
+// The rest of pass 1 for a CTA that gave up a wait: NaN in place of the products of the batch of n
+// job tiles that it has and of all that it takes after it.
+__device__ __noinline__ void dg_inter_nothing(DgSmem& sm, int n, const InterJob* jobs, const GemmTile* tiles,
+                                              int ntiles, int take, const SlotPtrs& sp, unsigned int* sched) {
+  for (;;) {
+    for (int q = 0; q < 2 * n; q++) {
+      const DgRecord& X = sm.rec[q];
+      if (X.k > 0)
+        for (int e = threadIdx.x; e < X.rows * X.cols; e += kDgThreads)
+          X.s[e % X.rows + static_cast<int64_t>(X.lds) * (e / X.rows)] = CUDART_NAN;
+    }
+    const int first = dg_next(sched, &sm.slot, take);
+    if (first >= ntiles) return;
+    n = min(take, ntiles - first);
+    dg_inter_batch(sm, jobs, tiles, first, n, sp);
+  }
+}
+
+// The same of pass 2, from tile half t on; its tiles still meet at their counters.
+__device__ __noinline__ void dg_sum_nothing(DgSmem& sm, int t, const SumGroup* groups, const GemmTile* tiles,
+                                            int ntiles, double* partials, unsigned int* counters, const SlotPtrs& sp,
+                                            unsigned int* sched) {
+  for (; t < 2 * ntiles; t = dg_next(sched, &sm.slot, 1)) {
+    const GemmTile T = tiles[t >> 1];
+    const SumGroup G = groups[T.idx];
+    const int row0 = (T.pos >> 16) * 64, col0 = (T.pos & 0xffff) * 64, off = (t & 1) * kDgCols;
+    const int tm = min(64, G.m - row0), width = min(64, G.n - col0);
+    if (off >= width) continue;
+    bool last = true;  // and the tile's other half goes with it
+    if (T.nsplit > 1) {
+      const int TM = 16 * ((T.shape & 3) + 1), TN = 16 * (((T.shape >> 2) & 3) + 1);
+      double* part = partials + T.part + static_cast<int64_t>(T.split) * TM * TN + TM * off;
+      for (int e = threadIdx.x; e < tm * min(kDgCols, width - off); e += kDgThreads)
+        __stcg(part + e % tm + TM * (e / tm), CUDART_NAN);
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0)
+        sm.is_last = atomicAdd(counters + T.counter, 1u) ==
+                     static_cast<unsigned>(T.nsplit * ((width + kDgCols - 1) / kDgCols) - 1);
+      __syncthreads();
+      last = sm.is_last;
+      if (last && threadIdx.x == 0) counters[T.counter] = 0u;
+    }
+    double* O = const_cast<double*>(resolve<double>(sp, G.out)) + row0 + static_cast<int64_t>(G.ldo) * col0;
+    if (last)
+      for (int e = threadIdx.x; e < tm * width; e += kDgThreads)
+        O[e % tm + static_cast<int64_t>(G.ldo) * (e / tm)] = CUDART_NAN;
+  }
+}
+
 // Pass 1, `take` job tiles at a time.
+template <long long kPolls>
 __global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
     inter_digits_kernel(const InterJob* __restrict__ jobs, const GemmTile* __restrict__ tiles, int ntiles, int take,
                         SlotPtrs sp, unsigned int* sched, int* err) {
   extern __shared__ unsigned char dyn[];
   DgSmem& sm = *reinterpret_cast<DgSmem*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
   dg_setup(sm);
-  DgEngine E(sm);
+  DgEngine<kPolls> E(sm);
   for (;;) {
     const int first = dg_next(sched, &sm.slot, take);
     if (first >= ntiles) break;
     const int n = min(take, ntiles - first);
-    if (static_cast<int>(threadIdx.x) < 2 * n) {
-      const GemmTile T = tiles[first + (threadIdx.x >> 1)];
-      const InterJob J = jobs[T.idx];
-      const int row0 = (T.pos >> 16) * 64, col0 = (T.pos & 0xffff) * 64 + (threadIdx.x & 1) * kDgCols;
-      DgRecord d{};
-      d.rows = static_cast<int16_t>(min(64, J.m - row0));
-      d.cols = static_cast<int16_t>(min(kDgCols, J.n - col0));
-      d.k = d.cols > 0 ? J.k : 0;
-      if (d.cols > 0) {
-        d.l = resolve<double>(sp, J.l.ref) + (J.l.trans ? static_cast<int64_t>(J.l.ld) * row0 : row0);
-        d.r = resolve<double>(sp, J.r.ref) + (J.r.trans ? col0 : static_cast<int64_t>(J.r.ld) * col0);
-        d.s = sp.inter + J.off + row0 + static_cast<int64_t>(J.m) * col0;
-      }
-      d.alpha = 1.0;
-      d.lld = J.l.ld;
-      d.rld = J.r.ld;
-      d.lds = J.m;
-      d.ltrans = J.l.trans != 0;
-      d.rtrans = J.r.trans == 0;
-      sm.rec[threadIdx.x] = d;
-    }
-    __syncthreads();
+    dg_inter_batch(sm, jobs, tiles, first, n, sp);
     DgInterSource src{2 * n};
-    if (!dg_stream<true>(E, src)) break;
+    if (!dg_stream<true>(E, src)) {
+      dg_inter_nothing(sm, n, jobs, tiles, ntiles, take, sp, sched);
+      break;
+    }
   }
   dg_end(E, sched, err);
 }
 
 // Pass 2: the column halves of the tiles one after another; a tile at most 32 columns wide
 // has one.
+template <long long kPolls>
 __global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
     sum_digits_kernel(const SumGroup* __restrict__ groups, const SumItem* __restrict__ items,
                       const GemmTile* __restrict__ tiles, int ntiles, double* partials, unsigned int* counters,
@@ -774,7 +847,7 @@ __global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
   extern __shared__ unsigned char dyn[];
   DgSmem& sm = *reinterpret_cast<DgSmem*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
   dg_setup(sm);
-  DgEngine E(sm);
+  DgEngine<kPolls> E(sm);
   for (;;) {
     const int t = dg_next(sched, &sm.slot, 1);
     if (t >= 2 * ntiles) break;
@@ -785,9 +858,12 @@ __global__ void __launch_bounds__(kDgThreads, kDgCtasPerSm)
     if (tn <= 0) continue;
     E.clear();
     DgSumSource src{items, T.item0, T.item1, sp, sm, row0, col0, tm, tn};
-    if (!dg_stream<false>(E, src)) break;
-    const bool big = tm > 32, mine = DgEngine::row_of(big) < tm;
-    const int r = DgEngine::row_of(big), c0 = DgEngine::col_of(big), nout = big ? 8 : 4;
+    if (!dg_stream<false>(E, src)) {
+      dg_sum_nothing(sm, t, groups, tiles, ntiles, partials, counters, sp, sched);
+      break;
+    }
+    const bool big = tm > 32, mine = E.row_of(big) < tm;
+    const int r = E.row_of(big), c0 = E.col_of(big), nout = big ? 8 : 4;
     // items without an inner dimension: out += alpha op(R)
     if (mine)
       for (int it = T.item0; it < T.item1; it++) {
@@ -857,27 +933,27 @@ int dg_grid(int units) {
 }  // namespace
 
 cudaError_t launch_inter_digits(const InterJob* jobs, const GemmTile* tiles, int ntiles, const SlotPtrs& sp,
-                                unsigned int* sched, int* err, cudaStream_t stream) {
+                                unsigned int* sched, int* err, cudaStream_t stream, bool give_up) {
   if (ntiles <= 0) return cudaSuccess;
-  const cudaError_t e =
-      cudaFuncSetAttribute(inter_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
+  const auto kernel = give_up ? inter_digits_kernel<0> : inter_digits_kernel<kTcSpinLimit>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
   if (e != cudaSuccess) return e;
   const int grid = dg_grid(ntiles);
   // several batches a CTA, so that no CTA is left with a long one at the end
   const int take = std::max(1, std::min(kDgBatch / 2, ntiles / (4 * grid)));
-  inter_digits_kernel<<<grid, kDgThreads, kDgSmemBytes, stream>>>(jobs, tiles, ntiles, take, sp, sched, err);
+  kernel<<<grid, kDgThreads, kDgSmemBytes, stream>>>(jobs, tiles, ntiles, take, sp, sched, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_sum_digits(const SumGroup* groups, const SumItem* items, const GemmTile* tiles, int ntiles,
                               double* partials, unsigned int* counters, const SlotPtrs& sp, unsigned int* sched,
-                              int* err, cudaStream_t stream) {
+                              int* err, cudaStream_t stream, bool give_up) {
   if (ntiles <= 0) return cudaSuccess;
-  const cudaError_t e =
-      cudaFuncSetAttribute(sum_digits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
+  const auto kernel = give_up ? sum_digits_kernel<0> : sum_digits_kernel<kTcSpinLimit>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
   if (e != cudaSuccess) return e;
-  sum_digits_kernel<<<dg_grid(2 * ntiles), kDgThreads, kDgSmemBytes, stream>>>(groups, items, tiles, ntiles, partials,
-                                                                                counters, sp, sched, err);
+  kernel<<<dg_grid(2 * ntiles), kDgThreads, kDgSmemBytes, stream>>>(groups, items, tiles, ntiles, partials, counters, sp,
+                                                                  sched, err);
   return cudaGetLastError();
 }
 

@@ -42,8 +42,8 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, uint32_t 
 }
 
 // bounded wait for phase `parity` of the barrier; false when the limit was reached
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity) {
-  for (long long i = 0; i < kTcSpinLimit; i++)
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity, long long polls = kTcSpinLimit) {
+  for (long long i = 0; i < polls; i++)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }

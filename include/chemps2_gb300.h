@@ -218,7 +218,9 @@ int c2g_dmrg_heff_apply_noalloc(c2g_dmrg* d, int index, const double* x, double*
  * buffers of n doubles, FP64 (precision 0) or FP32 arithmetic (precision 1), for the
  * current MPS and operators. `stream` (a cudaStream_t, or NULL): the call is ordered after
  * the work already issued on it and that stream waits for y_dev, without a host
- * synchronisation; with NULL the call returns when y_dev is written. */
+ * synchronisation; with NULL the call returns when y_dev is written. Should a kernel give up a
+ * bounded wait, y_dev holds NaN; with a stream this call has returned C2G_OK by then, and the
+ * next one that synchronises fails. */
 int c2g_dmrg_heff_apply_device(c2g_dmrg* d, int index, const double* x_dev, double* y_dev, int64_t n, int precision,
                                void* stream);
 
@@ -255,9 +257,10 @@ int c2g_rayleigh_ritz_eig(int n, const double* mat, int warm, double* evals, dou
  * sum = sum_i alpha_i L_i R_i (added over `splits` ranges of i) for `count` pairs of blocks, m x k and
  * k x n, column-major and concatenated; trans & 1: the L_i are stored transposed, trans & 2:
  * the R_i. digits != 0: on the tensor cores (as exact products of digits); 0: on the FP64
- * pipe. All sizes at most 4096. */
+ * pipe. All sizes at most 4096. given_up (nullable): with digits, room for the products and
+ * the sum of a run before this one, on the same scratch, whose kernels give up every wait. */
 int c2g_two_pass_products(int digits, int m, int n, int k, int count, int trans, int splits, const double* l,
-                          const double* r, const double* alpha, double* products, double* sum);
+                          const double* r, const double* alpha, double* products, double* sum, double* given_up);
 /* No counterpart in the reference (a diagnostic): the free memory of `device` (< 0: the
  * calling thread's current device; cudaMemGetInfo) and the bytes in use from that
  * device's default stream-ordered pool (cudaMemPoolAttrUsedMemCurrent), where this

@@ -24,7 +24,7 @@ U = 2.0**-53
 SIZES = [(17, 17, 12), (31, 33, 16), (32, 32, 32), (33, 65, 33), (64, 31, 47), (47, 47, 64), (65, 20, 70), (21, 27, 100)]
 
 
-def products(l, r, alpha, trans=0, splits=1, digits=1):
+def products(l, r, alpha, trans=0, splits=1, digits=1, given_up=None):
     """l: count x m x k, r: count x k x n -> (products, their weighted sum)."""
     count, m, k = l.shape
     n = r.shape[2]
@@ -34,7 +34,7 @@ def products(l, r, alpha, trans=0, splits=1, digits=1):
     out, total = np.zeros((count, n, m)), np.zeros((n, m))
     c2g._check(c2g.load().c2g_two_pass_products(digits, m, n, k, count, trans, splits, c2g._dp(lf), c2g._dp(rf),
                                                 c2g._dp(np.ascontiguousarray(alpha, dtype=np.float64)), c2g._dp(out),
-                                                c2g._dp(total)))
+                                                c2g._dp(total), None if given_up is None else c2g._dp(given_up)))
     return out.transpose(0, 2, 1), total.T
 
 
