@@ -583,6 +583,12 @@ int c2g_dmrg_heff_apply_device(c2g_dmrg* d, int index, const double* x_dev, doub
     d->d->heff_apply_device(index, x_dev, y_dev, n, precision, stream);
   });
 }
+int c2g_dmrg_leave_given_up(c2g_dmrg* d) {
+  return guarded([&] {
+    NEED(d);
+    d->d->leave_given_up();
+  });
+}
 int c2g_dmrg_sectors(const c2g_dmrg* d, int boundary, int* out, int cap, int* count) {
   return guarded([&] {
     NEED(d);

@@ -1352,6 +1352,7 @@ void DMRG::heff_apply_device(const int index, const double* x_dev, double* y_dev
   if (!x_dev || !y_dev) throw std::invalid_argument("heff_apply_device: null buffer");
   if (index < 0 || index > L - 2) throw std::out_of_range("heff_apply_device: index");
   if (precision != 0 && precision != 1) throw std::invalid_argument("heff_apply_device: precision must be 0 or 1");
+  rt->check_device_error();  // of an earlier call on a stream, which returned before it was done
   HeffCache& c = heff_program(index, false);
   const int64_t veclen = c.S->size();
   if (n != veclen) throw std::invalid_argument("heff_apply_device: vector length differs from the two-site object size");
@@ -1363,6 +1364,8 @@ void DMRG::heff_apply_device(const int index, const double* x_dev, double* y_dev
   if (u) rt->signal_to(u);  // the caller's stream waits for y
   else rt->sync();
 }
+
+void DMRG::leave_given_up() { rt->leave_given_up(); }
 
 void DMRG::heff_apply_noalloc(const int index, const double* x, double* y, const long long n) {
   if (!x || !y) throw std::invalid_argument("heff_apply_noalloc: null buffer");

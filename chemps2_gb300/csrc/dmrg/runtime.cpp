@@ -1116,9 +1116,27 @@ void Runtime::check_device_error() {
   if (err_host_ && *err_host_ != 0) {
     const int e = *err_host_;
     *err_host_ = 0;
+    // the kernel may have left scheduler or arrival counters raised: a later product would add
+    // up split tiles before they are all there
+    C2G_CUDA(cudaMemsetAsync(sched_, 0, sizeof(unsigned int) * 4, stream_));
+    for (int k : {kTransientGemmCounters, kTransientCounters})
+      if (transient_[k])
+        C2G_CUDA(cudaMemsetAsync(transient_[k], 0, static_cast<size_t>(transient_cap_[k]), stream_));
     throw std::runtime_error("a tensor-core kernel gave up a bounded wait (device error word " + std::to_string(e) +
-                             "); its output tiles were not written");
+                             "); its output tiles are not valid");
   }
+}
+
+void Runtime::leave_given_up() {
+  sync();
+  for (int k : {kTransientGemmCounters, kTransientCounters}) {
+    const std::vector<unsigned> raised(static_cast<size_t>(transient_cap_[k]) / sizeof(unsigned), 1u);
+    if (transient_[k])
+      C2G_CUDA(cudaMemcpyAsync(transient_[k], raised.data(), sizeof(unsigned) * raised.size(), cudaMemcpyHostToDevice,
+                               stream_));
+    C2G_CUDA(cudaStreamSynchronize(stream_));
+  }
+  *err_host_ = 2;
 }
 
 cudaStream_t Runtime::aux_stream() {

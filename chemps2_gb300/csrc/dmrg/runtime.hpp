@@ -133,9 +133,12 @@ class Runtime {
 
   const double* ones(int64_t n);
   // Synchronises the runtime's streams, then throws if a kernel reported a failed bounded
-  // wait since the last check (the device error word is cleared).
+  // wait since the last check (the device error word and all counters are cleared).
   void sync();
   void check_device_error();
+  // For tests: leaves what a kernel that gave up a wait may leave, the error word set and the
+  // arrival counters of split tiles raised.
+  void leave_given_up();
 
   // Scratch for reductions and small Davidson quantities.
   double* partial() { return partial_; }

@@ -127,9 +127,12 @@ class DMRG {
   // Extension: y_dev = Heff x_dev on the caller's device buffers (precision 0: FP64, 1:
   // FP32 arithmetic). With a CUDA stream the call is ordered after the work already on it
   // and that stream waits for the result (no host synchronisation); without one the call
-  // returns when y_dev is written.
+  // returns when y_dev is written. On a stream, a product of which a kernel gave up a wait
+  // holds NaN, and the next call that synchronises or runs here throws.
   void heff_apply_device(const int index, const double* x_dev, double* y_dev, const long long n,
                          const int precision, void* stream);
+  // For tests: leaves on the device what a kernel that gave up a wait may leave.
+  void leave_given_up();
 
   // CheMPS2/DMRG.h calc2DMandCorrelations (CheMPS2/DMRGtechnics.cpp:40-262 without the
   // 3-RDM): the two-particle density matrix of the current state, one site at a time from

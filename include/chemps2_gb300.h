@@ -220,9 +220,12 @@ int c2g_dmrg_heff_apply_noalloc(c2g_dmrg* d, int index, const double* x, double*
  * the work already issued on it and that stream waits for y_dev, without a host
  * synchronisation; with NULL the call returns when y_dev is written. Should a kernel give up a
  * bounded wait, y_dev holds NaN; with a stream this call has returned C2G_OK by then, and the
- * next one that synchronises fails. */
+ * next one that synchronises or comes here fails. */
 int c2g_dmrg_heff_apply_device(c2g_dmrg* d, int index, const double* x_dev, double* y_dev, int64_t n, int precision,
                                void* stream);
+/* For testing: leaves on the device what a kernel that gave up a wait may leave (its error
+ * word set, arrival counters raised); the next call that synchronises fails and clears it. */
+int c2g_dmrg_leave_given_up(c2g_dmrg* d);
 
 /* ---- Batches of independent problems (no counterpart in the reference, whose callers
  * loop over problems with one CheMPS2::DMRG each, e.g. CheMPS2/CASSCFnewtonraphson.cpp:
