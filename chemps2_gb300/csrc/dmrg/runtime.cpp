@@ -96,10 +96,10 @@ Runtime::Runtime(int L, int device) : L_(L) {
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&dev_slots_), sizeof(double*) * kMaxSlots));
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&dev_slots32_), sizeof(float*) * kMaxSlots));
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&partial_), sizeof(double) * kDotScratch));
-  C2G_CUDA(cudaMemset(partial_, 0, sizeof(double) * kDotScratch));
+  C2G_CUDA(cudaMemsetAsync(partial_, 0, sizeof(double) * kDotScratch, stream_));
   // tile-scheduler counters of the persistent tensor-core kernels (two per kernel)
   C2G_CUDA(cudaMalloc(reinterpret_cast<void**>(&sched_), sizeof(unsigned int) * 4));
-  C2G_CUDA(cudaMemset(sched_, 0, sizeof(unsigned int) * 4));
+  C2G_CUDA(cudaMemsetAsync(sched_, 0, sizeof(unsigned int) * 4, stream_));
   C2G_CUDA(cudaMallocHost(reinterpret_cast<void**>(&pinned_), sizeof(double) * 8));
   // error word of the kernels with bounded waits, mapped so that the host reads it after
   // any synchronisation without a copy
