@@ -1,7 +1,8 @@
-// One-CTA symmetric eigensolvers (FP64 results): the Rayleigh-Ritz problem of the Davidson
-// solver (order <= 32) and the Gram matrices of the truncation (order <= 128), all by
-// cyclic Jacobi with the round-robin (Brent-Luk) ordering: n / 2 disjoint plane rotations a
-// round, n - 1 rounds a sweep.
+// Symmetric eigensolvers (FP64 results): the Rayleigh-Ritz problem of the Davidson solver
+// (order <= 32, one CTA) and the Gram matrices of the truncation (order <= 128, one CTA each, or
+// above order 32 a cluster of eight where they are few), all by cyclic Jacobi with the
+// round-robin (Brent-Luk) ordering: n / 2 disjoint plane rotations a round, n - 1 rounds a
+// sweep.
 //
 // What bounds them: a warp's FP64 instruction takes 65 clocks here, dependent or not, and an
 // SM does 1.6 FP64 multiply-adds a clock (both measured); an FP32 one takes 6, and an SM
@@ -304,8 +305,8 @@ __device__ __forceinline__ void load_v(int n, int m, double* V, const double* W)
 }
 
 // V (n columns of n, orthonormal to 1e-4 or better) orthonormalised, A = V^T G V for the
-// matrix sc G (n x n). W: n x n scratch.
-__device__ void orthonormal_transform(int n, int m, const double* G, double sc, double* A, double* V, double* W) {
+// matrix G (n x n). W: n x n scratch.
+__device__ void orthonormal_transform(int n, int m, const double* G, double* A, double* V, double* W) {
   __shared__ double diag[kBatchedEigLargeMax];
   const int tid = threadIdx.x, nt = blockDim.x, ld = v_ld(n);
   auto lower = [&](const double* X, int i, int j) { return i >= j ? X[i + n * j] : X[j + n * i]; };
@@ -335,7 +336,7 @@ __device__ void orthonormal_transform(int n, int m, const double* G, double sc, 
   __syncthreads();
   cta_product<false>(
       n, n, [&](int i, int k) { return G[i + n * k]; }, [&](int k, int j) { return V[k + ld * j]; },
-      [&](int i, int j, double v) { W[i + n * j] = sc * v; });
+      [&](int i, int j, double v) { W[i + n * j] = v; });
   cta_product<true>(
       n, n, [&](int i, int k) { return V[k + ld * i]; }, [&](int k, int j) { return W[k + n * j]; },
       [&](int i, int j, double v) { A[tri(i, j)] = v; });
@@ -350,13 +351,13 @@ constexpr float kTol32 = 1e-11f;
 constexpr int kSweeps32 = 12;
 constexpr int kPasses32 = 2;
 
-// The eigenproblem of sc G (n x n). In: A = V0^T G V0 packed, W = V0 (n x n, orthonormal) or, with
+// The eigenproblem of G (n x n). In: A = V0^T G V0 packed, W = V0 (n x n, orthonormal) or, with
 // `unit`, V0 = 1 and W not set. Out: the eigenvectors V (n x m, leading
 // dimension v_ld(n)) and A = V^T G V diagonal.
 // During an FP32 pass V's memory holds the FP32 eigenvectors and matrix, and W the FP64
 // eigenvectors, which are then multiplied by half their rows at a time through A's memory.
-__device__ void eigen(int n, int m, bool unit, const double* G, double sc, double* A, double* V, double* W, Planes<float>& shf,
-                      Planes<double>& sh) {
+__device__ void eigen(int n, int m, bool unit, const double* G, double* A, double* V, double* W,
+                      Planes<float>& shf, Planes<double>& sh) {
   const int tid = threadIdx.x, nt = blockDim.x;
   float* Vf = reinterpret_cast<float*>(V);
   float* Af = Vf + n * m;
@@ -385,7 +386,7 @@ __device__ void eigen(int n, int m, bool unit, const double* G, double sc, doubl
     }
     load_v(n, m, V, W);
     __syncthreads();
-    orthonormal_transform(n, m, G, sc, A, V, W);
+    orthonormal_transform(n, m, G, A, V, W);
     if (pass + 1 < kPasses32) {
       for (int e = tid; e < n * n; e += nt) W[e] = V[e % n + v_ld(n) * (e / n)];
       __syncthreads();
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) rr_eig_kernel(const double* __r
     __syncthreads();
   }
   if (n > 1) {
-    eigen(n, m, !warm, G, 1.0, A, V, W, shf, sh);
+    eigen(n, m, !warm, G, A, V, W, shf, sh);
   } else {
     if (tid == 0) V[0] = 1.0;
     __syncthreads();
@@ -539,10 +540,11 @@ __global__ void __launch_bounds__(kRrThreads, 1) rr_eig_kernel(const double* __r
   }
 }
 
-// The Gram matrices of the truncation, one CTA each, by FP64 sweeps throughout: a sector may
-// have to keep singular values far below 1e-8 of the largest, whose vectors the sweeps find
-// from the matrix's own small elements (which carry their own relative accuracy), while
-// V^T G V would round them to 1e-16 of the norm.
+// The Gram matrices of the truncation, one CTA each, by FP64 sweeps throughout: their rotations
+// leave a graded matrix's small elements their own relative accuracy, while V^T G V would
+// round them to 1e-16 of the norm. The sweeps end at an off-diagonal part of 1e-15 of the norm:
+// vectors of eigenvalues below that (singular values below 3e-8 of the largest) may still be
+// mixed with one another.
 __device__ __forceinline__ void gram_eigen(const EigJob& jb, double* base, double* A, double* V, Planes<double>& sh,
                                            int* order) {
   const int n = jb.n, m = even_up(n), ld = v_ld(n), tid = threadIdx.x, nt = blockDim.x;
@@ -596,11 +598,13 @@ __global__ void __launch_bounds__(kEigLargeThreads) batched_eig_large_kernel(con
 // arrival at the barrier and the wait. Now a round's chain bounds it (rotations from remote
 // elements, blocks, barrier: 1 to 5 us).
 constexpr int kCl = 8, kClThreads = 256;
-// While two of its CTAs fit an SM the cluster is the faster one; ms for one CTA -> cluster, Gaussian
-// spectrum: 6 matrices order 33 0.61 -> 0.52, 48 1.22 -> 0.77, 64 2.85 -> 1.21, 96 9.0 -> 2.7, 128
-// 20.3 -> 5.1; 38 matrices 0.55 -> 0.58, 1.23 -> 1.10, 2.86 -> 1.79, 9.0 -> 5.3, 20.9 -> 11.7; 60
-// matrices 0.55 -> 1.16, 1.24 -> 1.97, 2.85 -> 3.24, 8.6 -> 9.4, 20.6 -> 19.5. (512 threads: 4.8 ms for
-// one of order 128 instead of 5.2, but half as many at a time; four CTAs: 7.9 ms.)
+// The line is by the number of matrices alone, where two CTAs of the clusters come to an SM: up
+// to it the cluster loses at most 5 % (order 33), at 60 matrices one CTA each at most 5 % (order
+// 128). ms for one CTA -> cluster, Gaussian spectrum: 6 matrices order 33 0.61 -> 0.52, 48 1.22
+// -> 0.77, 64 2.85 -> 1.21, 96 9.0 -> 2.7, 128 20.3 -> 5.1; 38 matrices 0.55 -> 0.58, 1.23 -> 1.10,
+// 2.86 -> 1.79, 9.0 -> 5.3, 20.9 -> 11.7; 60 matrices 0.55 -> 1.16, 1.24 -> 1.97, 2.85 -> 3.24, 8.6 ->
+// 9.4, 20.6 -> 19.5. (512 threads: 4.8 ms for one of order 128 instead of 5.2, but half as many
+// at a time; four CTAs: 7.9 ms.)
 constexpr int kClMaxJobs = 38;
 constexpr int kClA = (tri_size(kBatchedEigLargeMax) + kCl - 1) / kCl;
 constexpr int kClRows = (kBatchedEigLargeMax + kCl - 1) / kCl, kClLd = kClRows + 1;

@@ -2,17 +2,18 @@
 //
 //   block sandwich     every term out += alpha sum_p ratio_p op(A_p) op(B) op(C_p) of a
 //                      task-program stage, by output tiles, in three variants: the team
-//                      kernel for tiles up to 16 x 16 (sandwich_warp.cuh), the two-pass GEMM path for large groups
-//                      (intermediates once, then split-K item sums; sandwich_gemm.cu,
-//                      in FP64 also sandwich_digits.cu on the tensor cores)
+//                      kernel for tiles up to 16 x 16 (sandwich_warp.cuh), the two-pass GEMM
+//                      path for large groups (intermediates once, then split-K item sums;
+//                      sandwich_gemm.cu, in FP64 also sandwich_digits.cu on the tensor cores)
 //                      and, for comparison only, the one-pass cooperative and
 //                      item-parallel kernels. Item sums run in a fixed order and split
 //                      tiles are reduced in split order, so results are deterministic.
 //   vector kernels     the Davidson eigensolver's dots, linear combinations and
-//                      preconditioner, with deterministic two-pass reductions.
-//   eigensolvers       one-CTA Jacobi (FP32 passes, FP64 finish; eig.cu) for the <= 32 x 32
-//                      Rayleigh-Ritz matrix, and batched for the truncation's Gram
-//                      matrices up to order 128.
+//                      preconditioner, with deterministic sums finished by the last CTA.
+//   eigensolvers       Jacobi (eig.cu): FP32 passes with an FP64 finish in one CTA for the
+//                      <= 32 x 32 Rayleigh-Ritz matrix; FP64 sweeps, batched, for the
+//                      truncation's Gram matrices up to order 128, in one CTA or a cluster
+//                      of eight each.
 #pragma once
 
 #include <cstdint>
@@ -247,10 +248,9 @@ struct EigJob {
   int64_t offG, offE, offU;
 };
 cudaError_t launch_batched_eig(const EigJob* jobs, int njobs, double* base, cudaStream_t stream);
-// The same for kBatchedEigMax < n <= kBatchedEigLargeMax: one 512-thread CTA per matrix with
-// the matrix and the eigenvectors in dynamic shared memory; the eigenvectors' slot (offU)
-// is scratch until they are written. nmax: the largest n among the jobs (sizes the shared
-// memory).
+// The same for kBatchedEigMax < n <= kBatchedEigLargeMax: a cluster of eight CTAs per matrix
+// where these are few, else one CTA with the matrix and the eigenvectors in dynamic shared
+// memory. nmax: the largest n among the jobs (sizes the shared memory).
 constexpr int kBatchedEigLargeMax = 128;
 cudaError_t launch_batched_eig_large(const EigJob* jobs, int njobs, int nmax, double* base, cudaStream_t stream);
 // u = V coef, t = HV coef - evals[0] u, out[0] = t . t

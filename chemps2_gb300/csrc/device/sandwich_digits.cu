@@ -32,7 +32,7 @@
 // L's digits are rows of shared memory digit by digit and so are R's columns, so that digit i
 // of L meets digits 0 .. 7 - i of R in one MMA whose accumulator starts at column group i: 8
 // MMAs of M = 128 for each 16 of K. Persistent 256-thread CTAs, two per SM (256 columns of
-// tensor memory and 110 KB of shared memory each, so that one cuts digits and rounds sums while the
+// tensor memory and 106 KB of shared memory each, so that one cuts digits and rounds sums while the
 // other's MMAs run) take the 64 x 32 halves of the tile lists' tiles from an atomic counter.
 // While the MMAs of a step run, all threads round the previous step's sums (copied from
 // tensor memory to shared memory by the warps of the quadrants that hold them) and the next
@@ -40,8 +40,8 @@
 // not cut again.
 //
 // What bounds it: a step's fixed chain, load - exponents - digits - MMA - collect, of 2.2 to
-// 4.6 us an SM whatever its size, with the tensor pipe busy a fifth to a quarter of the time and
-// the issue slots 35 to 40 %. us a product and SM, FP64 pipe -> digits, pass 1 / pass 2:
+// 4.6 us an SM whatever its size, with the tensor pipe busy 16 to 23 % of the time and the issue
+// slots 38 %. us a product and SM, FP64 pipe -> digits, pass 1 / pass 2:
 // 17 x 17 x 17 3.1 -> 2.7 / 4.2 -> 3.6, 32 x 32 x 32 8.3 -> 3.3 / 10.0 -> 4.6, 47 x 47 x 47 27 -> 11.0 /
 // 31 -> 11.7, 64 x 64 x 64 65 -> 14.8 / 73 -> 15.5. With seven digits and no weights the last three were
 // 3.0 / 4.4, 9.1 / 10.6 and 12.2 / 13.7, but outputs without a product near M lost up to all of their
@@ -952,8 +952,8 @@ cudaError_t launch_sum_digits(const SumGroup* groups, const SumItem* items, cons
   const auto kernel = give_up ? sum_digits_kernel<0> : sum_digits_kernel<kTcSpinLimit>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmemBytes);
   if (e != cudaSuccess) return e;
-  kernel<<<dg_grid(2 * ntiles), kDgThreads, kDgSmemBytes, stream>>>(groups, items, tiles, ntiles, partials, counters, sp,
-                                                                  sched, err);
+  kernel<<<dg_grid(2 * ntiles), kDgThreads, kDgSmemBytes, stream>>>(groups, items, tiles, ntiles, partials, counters,
+                                                                  sp, sched, err);
   return cudaGetLastError();
 }
 

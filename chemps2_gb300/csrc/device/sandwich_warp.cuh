@@ -256,10 +256,10 @@ __device__ __forceinline__ void run_tile(const WarpLaunch& w, const WarpTile& td
 // One kernel for all tile classes: the tiles of a stage run heaviest first whatever their
 // class, so a small chain's classes overlap instead of following one another (a launch of a
 // few tiles takes as long as its longest item chain) and a large one has a single tail.
-// Every class takes 126 to 168 registers, so no class loses residency to another. Against
-// one launch per row class: Hubbard L=8 D=64 matvec 132 -> 48 us, L=16 D=200 4.05 -> 3.75 ms,
-// C2v L=17 D=389 2.43 -> 1.82 ms, D2h L=24 D=1000 17.5 -> 14.5 ms, L=30 D=2000 145 -> 134 ms
-// (FP64) and 33.1 -> 28.8 ms (tensor-core form).
+// The kernel takes the registers of its largest class, 168, so three CTAs are resident on an SM
+// where the smallest class alone (126) would have four. Against one launch per row class: Hubbard
+// L=8 D=64 matvec 132 -> 48 us, L=16 D=200 4.05 -> 3.75 ms, C2v L=17 D=389 2.43 -> 1.82 ms, D2h L=24
+// D=1000 17.5 -> 14.5 ms, L=30 D=2000 145 -> 134 ms (FP64) and 33.1 -> 28.8 ms (tensor-core form).
 template <typename Real>
 __global__ void __launch_bounds__(kWT) sandwich_warp_kernel(const WarpLaunch w, SlotPtrs sp) {
   __shared__ double smem[kWBuf];

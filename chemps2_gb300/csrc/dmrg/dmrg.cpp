@@ -999,7 +999,7 @@ double DMRG::solve_site(const int index, const double dvdson_rtol, const double 
   }
   // Eigendecomposition of every Gram matrix (FP64): sectors up to kBatchedEigMax in one
   // batched Jacobi launch, those up to kBatchedEigLargeMax in a second one (all sectors
-  // of a launch at once, one CTA each), larger ones with cuSOLVER syevd.
+  // of a launch at once, one CTA or one cluster each), larger ones with cuSOLVER syevd.
   std::vector<c2g::EigJob> jobs;
   int nsmall = 0, nmax_large = 0;
   for (const auto& c : plan.centers)

@@ -35,15 +35,17 @@ int warp_slots(int cls) {
 
 // Whether a tile of PM x PN units of 16 x 16 is formed from digits on the tensor cores
 // (sandwich_digits.cu) in FP64 runs; `k`: the inner dimension, summed over `products`
-// products. A digit step costs about the same (2.1 to 4.3 us of an SM) whatever its size up
+// products. A digit step costs about the same (2.2 to 4.6 us of an SM) whatever its size up
 // to 64 x 32 x 32, the FP64 pipe 0.16 us (pass 1) to 0.2 us for each of PM PN k / 4: measured,
-// 32 x 32 tiles (17 x 17 to 32 x 32 blocks), us a product and SM: k = 8 1.7 against 2.1 (pass 1)
-// and 2.1 against 2.8 (pass 2), k = 17 3.1 against 2.4 and 4.2 against 3.3, 32 x 32 x 32 8.3
-// against 3.0 and 10.0 against 4.3, 64 x 64 x 64 65 against 12 and 73 against 14. So one tile
-// alone breaks even at PM PN k of about 45 for each column half of 32; whole matvecs, where
-// the tiles left to the FP64 pipe are few, do best with the line at 24 to 40 (L = 24 D2h
-// D = 1000 14.4, 13.8, 13.9, 14.1 ms at 0, 24, 40, 56; Hubbard L = 18 D = 400 10.1, 10.7, 10.7,
-// 10.8 ms, against 14.5 and 28.2 ms on the FP64 pipe alone).
+// 32 x 32 tiles (17 x 17 to 32 x 32 blocks), us a product and SM: k = 8 1.7 against 2.2 (pass 1)
+// and 2.1 against 2.7 (pass 2), k = 17 3.1 against 2.7 and 4.2 against 3.6, 32 x 32 x 32 8.3
+// against 3.3 and 10.0 against 4.6, 64 x 64 x 64 65 against 15 and 73 against 16. So one tile
+// alone breaks even at PM PN k of about 45 for each column half of 32, and with the rest of the
+// matvec beside it a little lower. Whole matvecs with the line at 0, 16, 24, 32, 40, 56 and all
+// on the FP64 pipe, ms: Hubbard L = 16 D = 200 3.21, 3.20, 3.06, 2.98, 2.98, 3.10, 3.74; L = 18 D = 400
+// 13.5, 13.3, 13.5, 13.4, 13.7, 12.7, 28.1; L = 20 D = 512 33.1, 32.5, 33.2, 31.5, 31.5, 32.0, 60.7; C2v
+// L = 20 D = 800 17.8, 16.9, 16.8, 16.1, 16.3, 16.8, 20.3; D2h L = 24 D = 1000 15.0, 15.0, 13.8, 13.8,
+// 13.9, 14.4, 14.5; D2h L = 30 D = 2000 117, 114, 110, 108, 109, 109, 133.
 constexpr int64_t kDigitsLine = 32;
 bool digits_pay(int shape, int64_t k, int64_t products) {
   const int pm = (shape & 3) + 1, pn = ((shape >> 2) & 3) + 1;
